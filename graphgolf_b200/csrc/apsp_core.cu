@@ -25,6 +25,7 @@
 
 #include "../../include/graphgolf_b200.h"
 #include "apsp_kernel.cuh"
+#include "apsp_slice.cuh"
 #include "core_internal.h"
 
 namespace ggb {
@@ -141,6 +142,12 @@ struct State {
   long long* d_tll = nullptr;     // team_off [kMaxTeams], team_cells [kMaxTeams]
   unsigned char* h_team = nullptr;   // pinned: the above for upload, then results for read-back
   int last_teams = 0;
+  // shared-memory windows (apsp_slice.cuh)
+  ApspCtrl* d_sctrl = nullptr;       // all zero between launches
+  ApspCtrl* h_sout = nullptr;        // pinned: the result record the kernel writes
+  unsigned* d_packed = nullptr; size_t cap_packed = 0;   // the 16-bit rows of a lattice
+  unsigned* d_diff = nullptr;        // lattice_prep_kernel's differences and the height
+  bool last_slice = false;
   // last launch bookkeeping (for ggb_collect)
   int last_N = 0, last_R = 0, last_W = 0;
   bool pending = false;
@@ -214,6 +221,12 @@ const void* team_kernel_for(int R) {
   }
 }
 
+constexpr int kSliceStatic = 1024;   // static shared memory of slice_kernel, rounded up
+
+const void* slice_kernel_for(int words) {
+  return words == 1 ? (const void*)ggb::slice_kernel<1> : (const void*)ggb::slice_kernel<2>;
+}
+
 int ensure_ready(int device) {
   if (g.ready) return GGB_OK;
   if (device < 0) {
@@ -252,6 +265,11 @@ int ensure_ready(int device) {
                                 smem_optin - 4096));
   CUDA_TRY(cudaFuncSetAttribute((const void*)ggb::ball_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 smem_optin - 4096));
+  CUDA_TRY(cudaMalloc(&g.d_sctrl, sizeof(ApspCtrl)));
+  CUDA_TRY(cudaMemset(g.d_sctrl, 0, sizeof(ApspCtrl)));
+  CUDA_TRY(cudaHostAlloc(&g.h_sout, sizeof(ApspCtrl), cudaHostAllocDefault));
+  for (const void* k : {slice_kernel_for(1), slice_kernel_for(2), (const void*)ggb::slice_push_kernel})
+    CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - kSliceStatic));
   if (const char* s = getenv("GGB_BARRIER_TIMEOUT_NS")) g.timeout_ns = atoll(s);
   g.ready = true;
   return GGB_OK;
@@ -396,8 +414,161 @@ int launch_teams(const int* d_adj, int N, int d, int n_src1, int groups, int ran
   return GGB_OK;
 }
 
+// ---- shared-memory windows (apsp_slice.cuh) ------------------------------------
+
+// Whether any test hook or forced plan asks for the persistent kernel.
+bool slices_allowed() {
+  return !g.force_R && !g.force_ctas && !g.phantom && !g.trace_cap && g.ball_mode == -1;
+}
+
+struct SlicePlan {
+  int words = 0;      // 32-bit words per row (0: not served)
+  int threads = 0, grid = 0;
+  size_t smem = 0;
+};
+
+// A window is one CTA's work here and the whole GPU's in the persistent
+// kernel, so slices pay while every window has an SM to itself and a level's
+// gathers, N * (d + 1) of them, cost less than the grid barriers they replace.
+// Measured (kernel us, slices against persistent): N * (d + 1) = 32 900 (4700,
+// d = 6) 39 / 48; 42 624 (4736, d = 8) 37 / 44; 44 000 (4000, d = 10) 35 / 36;
+// 73 728 (8192, d = 8, 8 groups) 49 / 34.  Rows of 64 sources serve sparse
+// graphs that 32 would give more windows than SMs: 47 000 (9400, d = 4)
+// 74 / 170, against 100 with 32.
+SlicePlan plan_slice(int N, int d, int n_src1, int ac) {
+  SlicePlan p;
+  const long long gathers = (long long)N * (d + 1);
+  if (!slices_allowed() || N > ggb::kSliceMaxN || gathers > 47000) return p;
+  const int np = (N + 31) / 32 * 32, pairs = (d + 1) / 2;
+  for (int words = 1; words <= 2; ++words) {
+    const int w = 32 * words;
+    const int nw = (n_src1 + w - 1) / w + (ac + w - 1) / w;
+    const size_t smem = ggb::slice_smem_bytes(np, words, pairs);
+    if (nw > g.sms || smem > (size_t)(g.smem_optin - kSliceStatic)) continue;
+    p.words = words;
+    p.threads = std::min(1024, np);
+    p.smem = smem;
+    p.grid = nw;
+    return p;
+  }
+  return p;
+}
+
+void launched_slices(int N, int width) {
+  g.ev_ball = false;
+  g.last_N = N;
+  g.last_R = 0;
+  g.last_W = width;
+  g.last_teams = 0;
+  g.last_slice = true;
+  g.pending = true;
+}
+
+ggb::SliceArgs slice_args(int N, int d, int n_src1, int split, int ac, int groups, int width) {
+  ggb::SliceArgs a;
+  a.adj = nullptr;
+  a.adj16 = nullptr;
+  a.deg = nullptr;
+  a.ctrl = g.d_sctrl;
+  a.out = g.h_sout;
+  a.N = N;
+  a.d = d;
+  a.pairs = (d + 1) / 2;
+  a.np = (N + 31) / 32 * 32;
+  a.n_src1 = n_src1;
+  a.split = split;
+  a.ac = ac;
+  a.groups = groups;
+  a.width = width;
+  a.nw1 = (n_src1 + width - 1) / width;
+  a.nw2 = (ac + width - 1) / width;
+  a.dp = std::max(4, (d + 3) / 4 * 4);
+  a.height = nullptr;
+  return a;
+}
+
+// Whole evaluation on shared-memory windows.  The ids come as ints or,
+// straight from an upload, as 16 bits; deg as in SliceArgs.
+int launch_slice(const SlicePlan& pl, const int* d_adj, const uint16_t* d_adj16, const int* deg, int N, int d,
+                 int n_src1, int split, int ac, int groups, cudaStream_t st) {
+  ggb::SliceArgs a = slice_args(N, d, n_src1, split, ac, groups, 32 * pl.words);
+  a.adj = d_adj;
+  a.adj16 = d_adj16;
+  a.deg = deg;
+  if (g.timing) CUDA_TRY(cudaEventRecord(g.ev[0], st));
+  if (g.timing) CUDA_TRY(cudaEventRecord(g.ev[1], st));
+  if (pl.words == 1)
+    ggb::slice_kernel<1><<<pl.grid, pl.threads, pl.smem, st>>>(a);
+  else
+    ggb::slice_kernel<2><<<pl.grid, pl.threads, pl.smem, st>>>(a);
+  CUDA_TRY(cudaGetLastError());
+  ++g_launches;
+  if (g.timing) CUDA_TRY(cudaEventRecord(g.ev[2], st));
+  launched_slices(N, a.width);
+  return GGB_OK;
+}
+
+// A lattice graph whose rows fit: see launch_lattice.
+bool lattice_fits(int N) {
+  return slices_allowed() && ggb::slice_push_smem_bytes((N + 31) / 32 * 32) <= (size_t)(g.smem_optin - kSliceStatic);
+}
+
+// Grid evaluation on shared-memory windows: relabel and pack the rows, check
+// the relabel, read the lattice's height off the numbering, then every window
+// in one launch.  The uploaded ids are in d_adj16 or d_adj, rotate_hash in
+// d_rh and the degrees of a non-regular grid in d_deg.
+int launch_lattice(bool ids16, bool with_deg, int N, int d, int n_src1, int groups, cudaStream_t st) {
+  const int np = (N + 31) / 32 * 32, width = 32;
+  ggb::SliceArgs a = slice_args(N, d, n_src1, N, 0, groups, width);
+  const size_t row_words = ((size_t)N * a.dp + 1) / 2;
+  int rc = grow_device(&g.d_packed, &g.cap_packed, row_words);
+  if (rc) return rc;
+  if (!g.d_diff) {   // differences (zero between launches), then the height
+    CUDA_TRY(cudaMalloc(&g.d_diff, (ggb::kSliceMaxN / 32 + 1) * sizeof(unsigned)));
+    CUDA_TRY(cudaMemset(g.d_diff, 0, (ggb::kSliceMaxN / 32 + 1) * sizeof(unsigned)));
+  }
+  int* const height = reinterpret_cast<int*>(g.d_diff + ggb::kSliceMaxN / 32);
+  uint16_t* const rows = reinterpret_cast<uint16_t*>(g.d_packed);
+  CUDA_TRY(cudaMemsetAsync(g.d_inv, 0xff, (size_t)N * sizeof(int), st));
+  if (g.timing) CUDA_TRY(cudaEventRecord(g.ev[0], st));
+  if (g.timing) CUDA_TRY(cudaEventRecord(g.ev[1], st));
+  const int threads = 64, blocks = (N + threads - 1) / threads;
+  const int* deg = with_deg ? g.d_deg : nullptr;
+  if (ids16)
+    ggb::lattice_prep_kernel<uint16_t><<<blocks, threads, 0, st>>>(g.d_adj16, g.d_rh, deg, rows, g.d_inv, g.d_diff, N,
+                                                                  d, a.dp, a.ctrl);
+  else
+    ggb::lattice_prep_kernel<int><<<blocks, threads, 0, st>>>(g.d_adj, g.d_rh, deg, rows, g.d_inv, g.d_diff, N, d,
+                                                             a.dp, a.ctrl);
+  CUDA_TRY(cudaGetLastError());
+  ggb::lattice_height_kernel<<<1, 1024, 0, st>>>(g.d_inv, g.d_diff, N, n_src1, height, a.ctrl);
+  CUDA_TRY(cudaGetLastError());
+  a.adj16 = rows;
+  a.height = height;
+  // Small lattices take every vertex at every level (measured, us: 30 x 30
+  // degree 4 42 against 48 with rings, 40 x 50 degree 6 71 / 73, 60 x 60 degree
+  // 4 98 / 91).
+  if ((long long)N * (d + 1) <= 15000) {
+    a.d = a.dp;
+    a.pairs = a.dp / 2;
+    ggb::slice_kernel<1><<<std::min(a.nw1, g.sms), std::min(1024, np), ggb::slice_smem_bytes(np, 1, a.pairs), st>>>(a);
+  } else {
+    ggb::slice_push_kernel<<<std::min(a.nw1, g.sms), std::min(1024, np), ggb::slice_push_smem_bytes(np), st>>>(a);
+  }
+  CUDA_TRY(cudaGetLastError());
+  g_launches += 3;
+  if (g.timing) CUDA_TRY(cudaEventRecord(g.ev[2], st));
+  launched_slices(N, width);
+  return GGB_OK;
+}
+
 int launch_apsp(const int* d_adj, int N, int d, int n_src1, int split, int ac, int groups,
                 int rank, int procs, cudaStream_t st, const int* d_adj2 = nullptr) {
+  if (procs == 1 && !d_adj2) {
+    const SlicePlan pl = plan_slice(N, d, n_src1, ac);
+    if (pl.words) return launch_slice(pl, d_adj, nullptr, nullptr, N, d, n_src1, split, ac, groups, st);
+  }
+  g.last_slice = false;
   const int R = choose_R(N, d, std::max(n_src1, ac));
   const int ri = r_index(R);
   if (ri < 0) return fail(GGB_EINVAL, "window of %d uint4 per row is not supported", R);
@@ -577,10 +748,11 @@ int read_teams(cudaStream_t st, ggb_partial* p) {
 
 int read_ctrl(cudaStream_t st, ggb_partial* p) {
   if (g.last_teams > 0) return read_teams(st, p);
-  CUDA_TRY(cudaMemcpyAsync(g.h_ctrl, g.d_ctrl, sizeof(ApspCtrl), cudaMemcpyDeviceToHost, st));
+  if (!g.last_slice)   // slice_kernel writes its record to pinned memory itself
+    CUDA_TRY(cudaMemcpyAsync(g.h_ctrl, g.d_ctrl, sizeof(ApspCtrl), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
   g.pending = false;
-  const ApspCtrl& c = *g.h_ctrl;
+  const ApspCtrl& c = g.last_slice ? *g.h_sout : *g.h_ctrl;
   if (c.error == ggb::kErrAdj)
     return fail(GGB_EADJ, "adjacency entry outside [0, nodes) (reported by CTA/vertex %d)", c.error_info);
   if (c.error == ggb::kErrPerm)
@@ -635,7 +807,8 @@ int check_general(int nodes, int based_nodes, int groups, int degree, int added_
   return GGB_OK;
 }
 
-int stage_adj(const int* adj, size_t n, int nodes, cudaStream_t st) {
+// With kept16, ids that crossed as 16 bits stay in d_adj16 (*kept16 = true).
+int stage_adj(const int* adj, size_t n, int nodes, cudaStream_t st, bool* kept16 = nullptr) {
   int rc = grow_device(&g.d_adj, &g.cap_adj, n);
   if (rc) return rc;
   rc = grow_pinned(&g.h_adj, &g.cap_hadj, n);
@@ -650,7 +823,14 @@ int stage_adj(const int* adj, size_t n, int nodes, cudaStream_t st) {
   // The pinned copy must not be overwritten while a previous copy from it is
   // in flight: the stream is idle here (every host entry point waits).
   const ggb::StageSeg seg = {adj, 0, n};
-  CUDA_TRY(ggb::stage_upload_ids(g.device, g.h_adj, d16, g.d_adj, &seg, 1, n, st));
+  CUDA_TRY(ggb::stage_upload_ids(g.device, g.h_adj, d16, g.d_adj, &seg, 1, n, st, kept16));
+  return GGB_OK;
+}
+
+// Every degree of a non-regular graph lies in [0, max_degree].
+int check_degrees(const char* what, const int* deg, int nodes, int max_degree) {
+  for (int i = 0; i < nodes; ++i)
+    if ((unsigned)deg[i] > (unsigned)max_degree) return fail(GGB_EINVAL, "%s[%d] outside [0, max_degree]", what, i);
   return GGB_OK;
 }
 
@@ -710,6 +890,10 @@ void ggb_finalize(void) {
   cudaFreeHost(g.h_deg);
   cudaFree(g.d_bufs);
   cudaFree(g.d_ctrl);
+  cudaFree(g.d_sctrl);
+  cudaFreeHost(g.h_sout);
+  cudaFree(g.d_packed);
+  cudaFree(g.d_diff);
   cudaFree(g.d_trace);
   for (cudaEvent_t& e : g.ev)
     if (e) cudaEventDestroy(e);
@@ -830,8 +1014,15 @@ int ggb_eval_general_partial(int nodes, int based_nodes, int groups, int degree,
   if (rc) return rc;
   rc = ensure_ready(-1);
   if (rc) return rc;
-  rc = stage_adj(adj, (size_t)nodes * degree, nodes, g.stream);
+  const SlicePlan pl = procs == 1 ? plan_slice(nodes, degree, based_nodes, added_centers) : SlicePlan();
+  bool ids16 = false;
+  rc = stage_adj(adj, (size_t)nodes * degree, nodes, g.stream, pl.words ? &ids16 : nullptr);
   if (rc) return rc;
+  if (pl.words) {
+    rc = launch_slice(pl, ids16 ? nullptr : g.d_adj, ids16 ? g.d_adj16 : nullptr, nullptr, nodes, degree,
+                      based_nodes, based_nodes * groups, added_centers, groups, g.stream);
+    return rc ? rc : read_ctrl(g.stream, out);
+  }
   rc = launch_apsp(g.d_adj, nodes, degree, based_nodes, based_nodes * groups, added_centers, groups,
                    rank, procs, g.stream);
   if (rc) return rc;
@@ -956,17 +1147,27 @@ int eval_grid_impl(int nodes, int degree, const int* deg, int groups, const int*
   if ((long long)nodes * degree > INT_MAX) return fail(GGB_EINVAL, "nodes*degree too large");
   int rc = ensure_ready(-1);
   if (rc) return rc;
+  if (deg && (rc = check_degrees("degree", deg, nodes, degree))) return rc;
   const size_t n = (size_t)nodes * degree;
   cudaStream_t st = g.stream;
-  rc = stage_adj(adj, n, nodes, st);
+  const bool lattice = lattice_fits(nodes);
+  bool ids16 = false;
+  rc = stage_adj(adj, n, nodes, st, lattice ? &ids16 : nullptr);
   if (rc) return rc;
-  if ((rc = grow_device(&g.d_adj2, &g.cap_adj2, n))) return rc;
+  if (!lattice && (rc = grow_device(&g.d_adj2, &g.cap_adj2, n))) return rc;
   if ((rc = grow_device(&g.d_rh, &g.cap_rh, (size_t)nodes))) return rc;
   if ((rc = grow_device(&g.d_inv, &g.cap_inv, (size_t)nodes))) return rc;
   if ((rc = grow_pinned(&g.h_rh, &g.cap_hrh, (size_t)nodes))) return rc;
   if (deg && (rc = stage_deg(deg, (size_t)nodes, st))) return rc;
   std::memcpy(g.h_rh, rotate_hash, (size_t)nodes * sizeof(int));
   CUDA_TRY(cudaMemcpyAsync(g.d_rh, g.h_rh, (size_t)nodes * sizeof(int), cudaMemcpyHostToDevice, st));
+  if (lattice) {
+    if ((rc = launch_lattice(ids16, deg != nullptr, nodes, degree, based_nodes, groups, st))) return rc;
+    g.last_grid = true;
+    ggb_partial p;
+    if ((rc = read_ctrl(st, &p))) return rc;
+    return ggb_finish_grid(nodes, &p, out);
+  }
   CUDA_TRY(cudaMemsetAsync(g.d_ctrl, 0, sizeof(ApspCtrl), st));
   CUDA_TRY(cudaMemsetAsync(g.d_inv, 0xff, (size_t)nodes * sizeof(int), st));
   const int threads = 256;
@@ -1018,10 +1219,24 @@ int ggb_eval_general_nonregular(int nodes, int based_nodes, int groups, int max_
   if (rc) return rc;
   rc = ensure_ready(-1);
   if (rc) return rc;
+  if ((rc = check_degrees("num_degrees", num_degrees, nodes, max_degree))) return rc;
   const size_t n = (size_t)nodes * max_degree;
   cudaStream_t st = g.stream;
-  rc = stage_adj(adj, n, nodes, st);
+  // the added-centre phase gathers whole rows: one adjacency per phase
+  const SlicePlan pl = added_centers == 0 ? plan_slice(nodes, max_degree, based_nodes, 0) : SlicePlan();
+  bool ids16 = false;
+  rc = stage_adj(adj, n, nodes, st, pl.words ? &ids16 : nullptr);
   if (rc) return rc;
+  if (pl.words) {
+    if ((rc = stage_deg(num_degrees, (size_t)nodes, st))) return rc;
+    rc = launch_slice(pl, ids16 ? nullptr : g.d_adj, ids16 ? g.d_adj16 : nullptr, g.d_deg, nodes, max_degree,
+                      based_nodes, based_nodes * groups, 0, groups, st);
+    if (rc) return rc;
+    g.last_grid = false;
+    ggb_partial p;
+    if ((rc = read_ctrl(st, &p))) return rc;
+    return ggb_finish_general(nodes, &p, out);
+  }
   if ((rc = grow_device(&g.d_adj2, &g.cap_adj2, n))) return rc;
   if ((rc = stage_deg(num_degrees, (size_t)nodes, st))) return rc;
   CUDA_TRY(cudaMemsetAsync(g.d_ctrl, 0, sizeof(ApspCtrl), st));

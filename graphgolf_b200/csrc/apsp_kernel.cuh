@@ -67,6 +67,7 @@ struct ApspCtrl {
   int windows;
   int trace_len;                  // trace pairs written
   int done;                       // 1 once the outputs are written
+  int asym;                       // lattice graphs: some row's entry does not hold the row in return
 };
 
 struct ApspArgs {

@@ -42,9 +42,11 @@ cudaError_t stage_upload(int device, int* pinned, int* dev, const StageSeg* segs
 // Like stage_upload(), but when dev16 is given and every int lies in
 // [0, 65535], sends the ids as 16-bit values into dev16 and widens them into
 // dev on the device (one kernel launch on st).  Otherwise sends the ints as
-// they are.  Either way dev ends up holding exactly the caller's ints.
+// they are.  Either way dev ends up holding exactly the caller's ints.  With
+// kept16 given, ids that were sent as 16 bits stay in dev16 only (*kept16 =
+// true, dev is not written).
 cudaError_t stage_upload_ids(int device, int* pinned, uint16_t* dev16, int* dev, const StageSeg* segs, int nsegs,
-                             size_t total, cudaStream_t st);
+                             size_t total, cudaStream_t st, bool* kept16 = nullptr);
 
 // Number of threads stage_upload() copies with, the caller included.
 int stage_threads();

@@ -344,7 +344,8 @@ cudaError_t stage_upload(int device, int* pinned, int* dev, const StageSeg* segs
 }
 
 cudaError_t stage_upload_ids(int device, int* pinned, uint16_t* dev16, int* dev, const StageSeg* segs, int nsegs,
-                             size_t total, cudaStream_t st) {
+                             size_t total, cudaStream_t st, bool* kept16) {
+  if (kept16) *kept16 = false;
   static const bool narrow_on = [] {
     const char* e = std::getenv("GGB_STAGE_NARROW");
     return !(e && e[0] == '0');
@@ -364,6 +365,10 @@ cudaError_t stage_upload_ids(int device, int* pinned, uint16_t* dev16, int* dev,
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return e;
     return stage_upload(device, pinned, dev, segs, nsegs, total, st);
+  }
+  if (kept16) {
+    *kept16 = true;
+    return cudaSuccess;
   }
   const int threads = 256;
   const long long blocks = std::min<long long>(((long long)total / 8 + threads - 1) / threads + 1, 148 * 8);
