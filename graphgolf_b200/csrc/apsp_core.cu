@@ -26,6 +26,7 @@
 #include "../../include/graphgolf_b200.h"
 #include "apsp_kernel.cuh"
 #include "apsp_slice.cuh"
+#include "apsp_sym.cuh"
 #include "core_internal.h"
 
 namespace ggb {
@@ -97,6 +98,7 @@ struct State {
   int device = -1;
   int sms = 0;
   size_t l2_bytes = 0;
+  size_t mem_bytes = 0;
   cudaStream_t stream = nullptr;
   // device buffers (grow-only)
   int* d_adj = nullptr;       size_t cap_adj = 0;     // ints
@@ -148,6 +150,11 @@ struct State {
   unsigned* d_packed = nullptr; size_t cap_packed = 0;   // the 16-bit rows of a lattice
   unsigned* d_diff = nullptr;        // lattice_prep_kernel's differences and the height
   bool last_slice = false;
+  // symmetric halves of large graphs (apsp_sym.cuh)
+  uint4* d_tri = nullptr;     size_t cap_tri = 0;        // uint4, the triangular store
+  unsigned long long* d_symcnt = nullptr; size_t cap_symcnt = 0;    // counters, then list_n
+  unsigned long long* d_symlist = nullptr; size_t cap_symlist = 0;  // the list, the hash keys, their levels
+  bool last_sym = false;
   // last launch bookkeeping (for ggb_collect)
   int last_N = 0, last_R = 0, last_W = 0;
   bool pending = false;
@@ -227,6 +234,10 @@ const void* slice_kernel_for(int words) {
   return words == 1 ? (const void*)ggb::slice_kernel<1> : (const void*)ggb::slice_kernel<2>;
 }
 
+const void* sym_kernel_for(int R) {
+  return R == 32 ? (const void*)ggb::apsp_sym_kernel<32> : (const void*)ggb::apsp_sym_kernel<64>;
+}
+
 int ensure_ready(int device) {
   if (g.ready) return GGB_OK;
   if (device < 0) {
@@ -244,8 +255,9 @@ int ensure_ready(int device) {
   CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
   if (!coop) return fail(GGB_ECUDA, "device %d does not support cooperative launch", device);
   CUDA_TRY(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
-  CUDA_TRY(cudaMalloc(&g.d_ctrl, sizeof(ApspCtrl)));
-  CUDA_TRY(cudaHostAlloc(&g.h_ctrl, sizeof(ApspCtrl), cudaHostAllocDefault));
+  // [1]: the persistent kernel behind a symmetric one
+  CUDA_TRY(cudaMalloc(&g.d_ctrl, 2 * sizeof(ApspCtrl)));
+  CUDA_TRY(cudaHostAlloc(&g.h_ctrl, 2 * sizeof(ApspCtrl), cudaHostAllocDefault));
   for (int R = 1; R <= 64; R *= 2) {
     int nb = 0;
     CUDA_TRY(cudaFuncSetAttribute(kernel_for(R), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_for(R)));
@@ -270,6 +282,15 @@ int ensure_ready(int device) {
   CUDA_TRY(cudaHostAlloc(&g.h_sout, sizeof(ApspCtrl), cudaHostAllocDefault));
   for (const void* k : {slice_kernel_for(1), slice_kernel_for(2), (const void*)ggb::slice_push_kernel})
     CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - kSliceStatic));
+  for (const void* k : {(const void*)ggb::sym_ball_kernel<1>, (const void*)ggb::sym_ball_kernel<4>})
+    CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 4096));
+  for (int R : {32, 64}) {
+    int nb = 0;
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sym_kernel_for(R), ggb::kThreads, 0));
+    if (nb < 1) return fail(GGB_ECUDA, "symmetric kernel cannot be resident");
+  }
+  size_t free_b = 0;
+  CUDA_TRY(cudaMemGetInfo(&free_b, &g.mem_bytes));
   if (const char* s = getenv("GGB_BARRIER_TIMEOUT_NS")) g.timeout_ns = atoll(s);
   g.ready = true;
   return GGB_OK;
@@ -562,13 +583,138 @@ int launch_lattice(bool ids16, bool with_deg, int N, int d, int n_src1, int grou
   return GGB_OK;
 }
 
+// ---- symmetric halves (apsp_sym.cuh) ---------------------------------------------
+
+struct SymPlan {
+  int R = 0;              // 0: not served
+  int stored = 0;
+  int ball_warps = 0, ball_ctas = 0;
+  size_t ball_smem = 0, ball_cells = 0, tri_cells = 0, bytes = 0;
+};
+
+// Half sweeps pay once there are windows enough to halve and the ball, d^3 ids
+// a vertex, is small against N.  Measured (us, halves against the persistent
+// kernel): d = 12, N = 8000 102 / 82, 11000 137 / 184; d = 32, N = 30000
+// 763 / 682, 65536 2141 / 3538; d = 24, N = 20000 352 / 449; d = 4, N = 16384
+// 398 / 282, 20000 399 / 443; d = 3 at no size.
+SymPlan plan_sym(int N, int d) {
+  SymPlan p;
+  if (!slices_allowed() || d < 4 || d > 32 || N < 11000 || (d < 6 && N < 20000) || N < 1.3 * d * d * d) return p;
+  // the widest windows win while a level's rows stay near L2's size (N = 65536,
+  // d = 8: 1568 us with 8192 sources, 1726 with 4096)
+  const int R = (long long)N * 64 * 16 <= (128LL << 20) ? 64 : 32;
+  const int W = 128 * R, nwin = (N + W - 1) / W;
+  // k*: the first level at which the list is expected to hold the unreached
+  // pairs with room to spare; a random graph's share of them is q_{k+1} = q_k^(d-1)
+  const double dd = d;
+  double q = 1.0 - std::min(1.0, dd * (dd - 1) * (dd - 1) / N);
+  int k = 3;
+  while (k < ggb::kSymFirst + 11 && (k < ggb::kSymFirst || 0.5 * N * N * q > ggb::kSymTarget / 4)) {
+    q = std::pow(q, dd - 1);
+    ++k;
+  }
+  p.stored = k - ggb::kSymFirst;
+  for (int i = 0; i < nwin; ++i) p.tri_cells += (size_t)(N - std::min(N, (i + 1) * W)) * R;
+  p.ball_cells = (size_t)nwin * N * R;
+  const size_t per_warp = (size_t)ggb::sym_ball_warp_u4(N, d) * sizeof(uint4);
+  int best = 0;
+  for (int w = ggb::kBallThreads / 32; w >= 1; --w) {
+    const size_t sm = per_warp * w;
+    if (sm > (size_t)(g.smem_optin - 4096)) continue;
+    const int c = (int)std::min<size_t>(3, ((size_t)g.smem_optin + 1024) / (sm + 1024));
+    if (c * w > best) { best = c * w; p.ball_warps = w; p.ball_ctas = c; p.ball_smem = sm; }
+  }
+  if (!best) return p;
+  p.bytes = sizeof(uint4) * (p.ball_cells + p.tri_cells * p.stored + 4 * (size_t)N * R);
+  // the workspace stays with the library: a quarter of the device at most
+  if (p.bytes > g.mem_bytes / 4) return p;
+  p.R = R;
+  return p;
+}
+
+int launch_sym(const SymPlan& pl, const int* d_adj, int N, int d, cudaStream_t st, bool* done) {
+  *done = false;
+  const size_t cells = (size_t)N * pl.R;
+  const size_t nl = ggb::kSymList, cnt_words = ggb::kSymCounters + (1 + ggb::kSymPasses + 1) / 2;
+  // without the memory the persistent kernel serves the graph
+  if (grow_device(&g.d_bufs, &g.cap_buf, 4 * cells) || grow_device(&g.d_ball, &g.cap_ball, pl.ball_cells) ||
+      grow_device(&g.d_tri, &g.cap_tri, pl.tri_cells * pl.stored) ||
+      grow_device(&g.d_symcnt, &g.cap_symcnt, cnt_words) || grow_device(&g.d_symlist, &g.cap_symlist, 3 * nl + nl / 4))
+    return GGB_OK;
+  const bool vec4 = d % 4 == 0 && ((uintptr_t)d_adj % 16) == 0;
+  const void* k = sym_kernel_for(pl.R);
+  ApspArgs a;
+  std::memset(&a, 0, sizeof a);
+  a.adj = d_adj;
+  a.buf0 = g.d_bufs;
+  a.buf1 = g.d_bufs + cells;
+  a.ctrl = g.d_ctrl;
+  a.timeout_ns = g.timeout_ns;
+  a.N = N;
+  a.d = d;
+  a.n_src1 = N;
+  a.split = N;
+  a.groups = 1;
+  a.win_stride = 1;
+  a.vec4 = vec4 ? 1 : 0;
+  a.skip_permille = 900;
+  ggb::SymArgs s;
+  s.ball = g.d_ball;
+  s.tri = g.d_tri;
+  s.tri_cells = pl.tri_cells;
+  s.stored = pl.stored;
+  s.cnt = g.d_symcnt;
+  s.list_n = reinterpret_cast<unsigned*>(g.d_symcnt + ggb::kSymCounters);
+  s.list = g.d_symlist;
+  s.hash = g.d_symlist + nl;
+  s.hlev = reinterpret_cast<unsigned char*>(g.d_symlist + 3 * nl);
+  CUDA_TRY(cudaMemsetAsync(g.d_symcnt, 0, cnt_words * sizeof(unsigned long long), st));
+  CUDA_TRY(cudaMemsetAsync(g.d_ctrl, 0, 2 * sizeof(ApspCtrl), st));
+  if (g.timing) CUDA_TRY(cudaEventRecord(g.ev[0], st));
+  const long long need = ((long long)N + pl.ball_warps - 1) / pl.ball_warps;
+  const int bgrid = (int)std::min<long long>(need, (long long)pl.ball_ctas * g.sms);
+  if (vec4)
+    ggb::sym_ball_kernel<4><<<bgrid, pl.ball_warps * 32, pl.ball_smem, st>>>(d_adj, N, d, pl.R, g.d_ball, s.cnt, g.d_ctrl);
+  else
+    ggb::sym_ball_kernel<1><<<bgrid, pl.ball_warps * 32, pl.ball_smem, st>>>(d_adj, N, d, pl.R, g.d_ball, s.cnt, g.d_ctrl);
+  CUDA_TRY(cudaGetLastError());
+  if (g.timing) CUDA_TRY(cudaEventRecord(g.ev[1], st));
+  void* params[] = {(void*)&a, (void*)&s};
+  CUDA_TRY(cudaLaunchCooperativeKernel(k, dim3(g.sms), dim3(ggb::kThreads), params, 0, st));
+  a.ctrl = g.d_ctrl + 1;
+  a.only_if = g.d_ctrl;
+  void* params2[] = {(void*)&a};
+  CUDA_TRY(cudaLaunchCooperativeKernel(kernel_for(pl.R), dim3(std::min(g.sms, max_ctas(pl.R))), dim3(ggb::kThreads),
+                                       params2, smem_for(pl.R), st));
+  g_launches += 3;
+  if (g.timing) CUDA_TRY(cudaEventRecord(g.ev[2], st));
+  g.ev_ball = true;
+  g.last_N = N;
+  g.last_R = pl.R;
+  g.last_W = 128 * pl.R;
+  g.last_teams = 0;
+  g.last_sym = true;
+  g.pending = true;
+  *done = true;
+  return GGB_OK;
+}
+
 int launch_apsp(const int* d_adj, int N, int d, int n_src1, int split, int ac, int groups,
-                int rank, int procs, cudaStream_t st, const int* d_adj2 = nullptr) {
+                int rank, int procs, cudaStream_t st, const int* d_adj2 = nullptr, bool lattice = false) {
   if (procs == 1 && !d_adj2) {
     const SlicePlan pl = plan_slice(N, d, n_src1, ac);
     if (pl.words) return launch_slice(pl, d_adj, nullptr, nullptr, N, d, n_src1, split, ac, groups, st);
   }
   g.last_slice = false;
+  g.last_sym = false;
+  if (procs == 1 && !d_adj2 && groups == 1 && ac == 0 && n_src1 == N && !lattice) {   // lattices have too many levels
+    const SymPlan sp = plan_sym(N, d);
+    bool done = false;
+    if (sp.R) {
+      int rc = launch_sym(sp, d_adj, N, d, st, &done);
+      if (rc || done) return rc;
+    }
+  }
   const int R = choose_R(N, d, std::max(n_src1, ac));
   const int ri = r_index(R);
   if (ri < 0) return fail(GGB_EINVAL, "window of %d uint4 per row is not supported", R);
@@ -749,10 +895,10 @@ int read_teams(cudaStream_t st, ggb_partial* p) {
 int read_ctrl(cudaStream_t st, ggb_partial* p) {
   if (g.last_teams > 0) return read_teams(st, p);
   if (!g.last_slice)   // slice_kernel writes its record to pinned memory itself
-    CUDA_TRY(cudaMemcpyAsync(g.h_ctrl, g.d_ctrl, sizeof(ApspCtrl), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaMemcpyAsync(g.h_ctrl, g.d_ctrl, (g.last_sym ? 2 : 1) * sizeof(ApspCtrl), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
   g.pending = false;
-  const ApspCtrl& c = g.last_slice ? *g.h_sout : *g.h_ctrl;
+  const ApspCtrl& c = g.last_slice ? *g.h_sout : g.h_ctrl[g.last_sym && g.h_ctrl[0].fallback ? 1 : 0];
   if (c.error == ggb::kErrAdj)
     return fail(GGB_EADJ, "adjacency entry outside [0, nodes) (reported by CTA/vertex %d)", c.error_info);
   if (c.error == ggb::kErrPerm)
@@ -894,6 +1040,9 @@ void ggb_finalize(void) {
   cudaFreeHost(g.h_sout);
   cudaFree(g.d_packed);
   cudaFree(g.d_diff);
+  cudaFree(g.d_tri);
+  cudaFree(g.d_symcnt);
+  cudaFree(g.d_symlist);
   cudaFree(g.d_trace);
   for (cudaEvent_t& e : g.ev)
     if (e) cudaEventDestroy(e);
@@ -1188,7 +1337,7 @@ int eval_grid_impl(int nodes, int degree, const int* deg, int groups, const int*
   if (g.h_ctrl->error != 0)
     return fail(GGB_EPERM, "rotate_hash is not a permutation of [0, nodes) (at %d)", g.h_ctrl->error_info);
   g.last_grid = true;
-  rc = launch_apsp(g.d_adj2, nodes, degree, based_nodes, nodes, 0, groups, 0, 1, st);
+  rc = launch_apsp(g.d_adj2, nodes, degree, based_nodes, nodes, 0, groups, 0, 1, st, nullptr, true);
   if (rc) return rc;
   ggb_partial p;
   rc = read_ctrl(st, &p);

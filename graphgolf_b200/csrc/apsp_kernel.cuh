@@ -67,7 +67,8 @@ struct ApspCtrl {
   int windows;
   int trace_len;                  // trace pairs written
   int done;                       // 1 once the outputs are written
-  int asym;                       // lattice graphs: some row's entry does not hold the row in return
+  int asym;                       // some row's entry does not hold the row in return
+  int fallback;                   // the symmetric kernel left the graph to the persistent kernel
 };
 
 struct ApspArgs {
@@ -116,6 +117,8 @@ struct ApspArgs {
   // The sweeps that set and read them are described at sweep_stamped.
   unsigned* stamps = nullptr;
   unsigned stamp_base = 0;
+  // When given, the persistent kernel runs only if only_if->fallback is set.
+  const ApspCtrl* only_if = nullptr;
 };
 
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
@@ -1319,6 +1322,7 @@ template <int R>
 __global__ void __launch_bounds__(kThreads, 1) apsp_persistent_kernel(const ApspArgs a) {
   __shared__ ApspSmem sm;
   extern __shared__ unsigned s_dyn[];   // per warp: neighbour ids [4][64], then rows [4][2][SROW]
+  if (a.only_if && ld_volatile_i32(&a.only_if->fallback) == 0) return;   // written before the launch
   if (threadIdx.x < 8) sm.seen[threadIdx.x >> 1][threadIdx.x & 1] = 0ULL;
   __syncthreads();
   unsigned long long bar_target = 0;
