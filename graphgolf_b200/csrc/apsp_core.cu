@@ -27,6 +27,7 @@
 #include "apsp_kernel.cuh"
 #include "apsp_slice.cuh"
 #include "apsp_sym.cuh"
+#include "apsp_levels.cuh"
 #include "core_internal.h"
 
 namespace ggb {
@@ -284,6 +285,8 @@ int ensure_ready(int device) {
     CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - kSliceStatic));
   for (const void* k : {(const void*)ggb::sym_ball_kernel<1>, (const void*)ggb::sym_ball_kernel<4>})
     CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 4096));
+  CUDA_TRY(cudaFuncSetAttribute((const void*)ggb::apsp_levels_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                smem_optin - 4096));
   for (int R : {32, 64}) {
     int nb = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sym_kernel_for(R), ggb::kThreads, 0));
@@ -594,12 +597,12 @@ struct SymPlan {
 
 // Half sweeps pay once there are windows enough to halve and the ball, d^3 ids
 // a vertex, is small against N.  Measured (us, halves against the persistent
-// kernel): d = 12, N = 8000 102 / 82, 11000 137 / 184; d = 32, N = 30000
-// 763 / 682, 65536 2141 / 3538; d = 24, N = 20000 352 / 449; d = 4, N = 16384
-// 398 / 282, 20000 399 / 443; d = 3 at no size.
+// kernel): d = 7, N = 20000 253 / 385; d = 32, N = 30000 763 / 682, 65536
+// 2141 / 3538; d = 24, N = 20000 352 / 449; d = 4, N = 16384 398 / 282, 20000
+// 399 / 443; d = 3 at no size.  Smaller graphs: see levels_served.
 SymPlan plan_sym(int N, int d) {
   SymPlan p;
-  if (!slices_allowed() || d < 4 || d > 32 || N < 11000 || (d < 6 && N < 20000) || N < 1.3 * d * d * d) return p;
+  if (!slices_allowed() || d < 4 || d > 32 || N < 18000 || (d < 6 && N < 20000) || N < 1.3 * d * d * d) return p;
   // the widest windows win while a level's rows stay near L2's size (N = 65536,
   // d = 8: 1568 us with 8192 sources, 1726 with 4096)
   const int R = (long long)N * 64 * 16 <= (128LL << 20) ? 64 : 32;
@@ -699,6 +702,67 @@ int launch_sym(const SymPlan& pl, const int* d_adj, int N, int d, cudaStream_t s
   return GGB_OK;
 }
 
+// ---- level by level over all sources (apsp_levels.cuh) ------------------------------
+
+// Past 8192 vertices the persistent kernel needs a second window; up to about
+// 18 000 the two N x N matrices and their transposes stay near L2's size.
+// Measured (whole call, us, level by level / half-sweep windows / persistent
+// kernel): N = 8500, d = 12 110 / - / 147; 12000, d = 12 135 / 143 / 180;
+// 12000, d = 32 124 / - / 216; 16384, d = 12 180 / 187 / 216; 18000, d = 12
+// 219 / 216; 22000, d = 16 229 / 247; 8192, d = 12 109 / - / 81.
+bool levels_served(int N, int d) {
+  return slices_allowed() && d >= 4 && d <= 32 && N > 8192 && N <= (d >= 16 ? 22000 : 18000);
+}
+
+int launch_levels(const int* d_adj, int N, int d, cudaStream_t st, bool* done) {
+  *done = false;
+  const int C = ggb::levels_pitch(N), R = 32;   // R: the persistent kernel behind it
+  const size_t cells = (size_t)N * C;
+  const size_t words = ggb::kLevelsListWords + (ggb::kLevelsCounters + 1) / 2;
+  // without the memory another path serves the graph
+  if (grow_device(&g.d_bufs, &g.cap_buf, 2 * cells) || grow_device(&g.d_symlist, &g.cap_symlist, words)) return GGB_OK;
+  ApspArgs a;
+  std::memset(&a, 0, sizeof a);
+  a.adj = d_adj;
+  a.buf0 = g.d_bufs;
+  a.buf1 = g.d_bufs + cells;
+  a.ctrl = g.d_ctrl;
+  a.timeout_ns = g.timeout_ns;
+  a.N = N;
+  a.d = d;
+  a.n_src1 = N;
+  a.split = N;
+  a.groups = 1;
+  a.win_stride = 1;
+  a.vec4 = d % 4 == 0 && ((uintptr_t)d_adj % 16) == 0;
+  a.skip_permille = 900;
+  const ggb::LevelsList ws = ggb::levels_list(g.d_symlist);
+  CUDA_TRY(cudaMemsetAsync(ws.counters, 0, ggb::kLevelsCounters * sizeof(unsigned), st));
+  CUDA_TRY(cudaMemsetAsync(g.d_ctrl, 0, 2 * sizeof(ApspCtrl), st));
+  if (g.timing) CUDA_TRY(cudaEventRecord(g.ev[0], st));
+  if (g.timing) CUDA_TRY(cudaEventRecord(g.ev[1], st));
+  void* params[] = {(void*)&a, (void*)&ws};
+  CUDA_TRY(cudaLaunchCooperativeKernel((const void*)ggb::apsp_levels_kernel, dim3(g.sms), dim3(ggb::kThreads), params,
+                                       ggb::levels_smem_bytes(N, d), st));
+  a.buf1 = g.d_bufs + (size_t)N * R;
+  a.ctrl = g.d_ctrl + 1;
+  a.only_if = g.d_ctrl;
+  void* params2[] = {(void*)&a};
+  CUDA_TRY(cudaLaunchCooperativeKernel(kernel_for(R), dim3(std::min(g.sms, max_ctas(R))), dim3(ggb::kThreads),
+                                       params2, smem_for(R), st));
+  g_launches += 2;
+  if (g.timing) CUDA_TRY(cudaEventRecord(g.ev[2], st));
+  g.ev_ball = false;
+  g.last_N = N;
+  g.last_R = R;
+  g.last_W = 128 * C;
+  g.last_teams = 0;
+  g.last_sym = true;
+  g.pending = true;
+  *done = true;
+  return GGB_OK;
+}
+
 int launch_apsp(const int* d_adj, int N, int d, int n_src1, int split, int ac, int groups,
                 int rank, int procs, cudaStream_t st, const int* d_adj2 = nullptr, bool lattice = false) {
   if (procs == 1 && !d_adj2) {
@@ -708,8 +772,12 @@ int launch_apsp(const int* d_adj, int N, int d, int n_src1, int split, int ac, i
   g.last_slice = false;
   g.last_sym = false;
   if (procs == 1 && !d_adj2 && groups == 1 && ac == 0 && n_src1 == N && !lattice) {   // lattices have too many levels
-    const SymPlan sp = plan_sym(N, d);
     bool done = false;
+    if (levels_served(N, d)) {
+      int rc = launch_levels(d_adj, N, d, st, &done);
+      if (rc || done) return rc;
+    }
+    const SymPlan sp = plan_sym(N, d);
     if (sp.R) {
       int rc = launch_sym(sp, d_adj, N, d, st, &done);
       if (rc || done) return rc;

@@ -35,15 +35,17 @@
 // otherwise, evaluates the graph.
 //
 // Measured (whole call, us, against the persistent kernel with its ball):
-// N = 65536, d = 16 1262 / 1836 (ball 271 / 380, sweeps 955 / 1425); d = 8
-// 1568 / 2312; N = 16384, d = 12 182 / 216; N = 100000, d = 12 3240 / 6930;
+// N = 65536, d = 16 1218 / 1836 (ball 271 / 380, sweeps 910 / 1425); d = 8
+// 1528 / 2312; N = 16384, d = 12 182 / 216; N = 100000, d = 12 3240 / 6930;
 // N = 262144, d = 12 30 900 / 67 900.  Bound: L2 gathers, at 7 to 10 TB/s (the
 // persistent kernel's sweeps reach 13: half of the rows of a level lie in the
 // store, and the ball is read from HBM), and for the ball the load/store pipe
 // (91 % busy).  Tried and not kept: S_3 in halves too (the ball kernel 9 %
 // faster, its transposes cost more), sweeps that write every row twice instead
 // of choosing between two places (4 % slower), a prefetch of the next window's
-// ball slice into L2 (2 % slower), windows of 1024 to 2048 sources.
+// ball slice into L2 (2 % slower), windows of 1024 to 2048 sources, 768 or 1024
+// threads with 6 or 4 neighbour rows in flight (10 to 20 % slower), half a warp
+// per 1 KB row with two parts a lane (5 % slower).
 #pragma once
 #include "apsp_kernel.cuh"
 
@@ -230,7 +232,8 @@ __device__ __forceinline__ void transpose_tile(const uint4* __restrict__ src, si
 // ---- one half sweep -----------------------------------------------------------------
 // Appends the unset bits among the `nv` valid ones of word `x` (bit b is
 // source s0 + b) of row v; in the diagonal block only sources below v.
-__device__ __forceinline__ void list_missing(const SymArgs& s, unsigned x, int nv, int v, int s0, bool diag) {
+__device__ __forceinline__ void list_missing(const SymArgs& s, unsigned x, int nv, int v, int s0, bool diag,
+                                             unsigned cap = kSymList) {
   unsigned m = ~x & (nv >= 32 ? 0xffffffffu : (1u << max(nv, 0)) - 1u);
   if (diag) {
     const int b = v - s0;                       // sources s0 .. v - 1
@@ -241,7 +244,7 @@ __device__ __forceinline__ void list_missing(const SymArgs& s, unsigned x, int n
   while (m) {
     const int b = __ffs(m) - 1;
     m &= m - 1;
-    if (at < kSymList) s.list[at] = ((unsigned long long)(unsigned)v << 32) | (unsigned)(s0 + b);
+    if (at < cap) s.list[at] = ((unsigned long long)(unsigned)v << 32) | (unsigned)(s0 + b);
     ++at;
   }
 }
@@ -268,7 +271,7 @@ __device__ __forceinline__ void sym_sweep(const SymArgs& s, const SymRows src, u
                                           uint4* __restrict__ hi, const int* __restrict__ adj, int N, int d, int vec4,
                                           int first, int v_next, int l, bool early, long long warp_id,
                                           long long n_warps, unsigned& c_diag, unsigned& c_off) {
-  constexpr int LP = R / 2 < 16 ? R / 2 : 16;     // lanes a row
+  constexpr int LP = R / 2 < 32 ? R / 2 : 32;     // lanes a row
   constexpr int PPL = R / (2 * LP);               // 32-byte parts a lane
   constexpr int G = 32 / LP;                      // rows a warp and step
   constexpr int U = 8 / PPL;                      // neighbour rows in flight
@@ -417,7 +420,7 @@ __device__ __forceinline__ bool grid_wait(ApspCtrl* c, unsigned long long target
 template <int R>
 __device__ __forceinline__ void sym_list_window0(const SymArgs& s, const SymRows rows, int N, int l,
                                                  long long warp_id, long long n_warps) {
-  constexpr int LP = R / 2 < 16 ? R / 2 : 16, PPL = R / (2 * LP), G = 32 / LP;
+  constexpr int LP = R / 2 < 32 ? R / 2 : 32, PPL = R / (2 * LP), G = 32 / LP;
   const int lane = threadIdx.x & 31, h = lane / LP, hl = lane % LP;
   for (long long vb = warp_id * G; vb + h < N; vb += n_warps * G) {
     const int v = (int)(vb + h);
@@ -429,6 +432,74 @@ __device__ __forceinline__ void sym_list_window0(const SymArgs& s, const SymRows
       if (nv > 0 && popc4(x[0]) + popc4(x[1]) != (unsigned)nv)
         for (int k = 0; k < 8; ++k) list_missing(s, word_of(x, k), nv - 32 * k, v, b0 + 32 * k, v < l);
     }
+  }
+}
+
+enum : int { kSymFailed = 0, kSymResolved = 1, kSymStalled = 2, kSymTooLong = 3 };
+
+// Resolves the n > 0 listed pairs, unreached at level k, level by level on the
+// `nt` threads of a team (this one is number tid): pass p makes level k + 1 + p.
+// late receives twice the sum of the unreached pairs at levels k, k + 1, ...,
+// passes the levels it took; left[p] (zeroed) the pairs left after pass p.
+template <typename Barrier>
+__device__ __forceinline__ int sym_resolve(const SymArgs& s, unsigned* left, const int* __restrict__ adj, int d,
+                                           unsigned n, int max_passes, unsigned tid, unsigned nt, Barrier barrier,
+                                           unsigned long long& late, int& passes) {
+  unsigned size = 1024;
+  while (size < 2 * n) size <<= 1;
+  const unsigned mask = size - 1;
+  for (unsigned i = tid; i < size; i += nt) {
+    __stcg(s.hash + i, kSymEmpty);
+    s.hlev[i] = 255;
+  }
+  if (!barrier()) return kSymFailed;
+  auto key_of_pair = [](unsigned x, unsigned y) {
+    return x > y ? ((unsigned long long)x << 32) | y : ((unsigned long long)y << 32) | x;
+  };
+  for (unsigned i = tid; i < n; i += nt) {
+    const unsigned long long e = __ldcg(s.list + i);
+    const unsigned long long key = key_of_pair((unsigned)(e >> 32), (unsigned)e);
+    unsigned h = sym_slot(key) & mask;
+    while (atomicCAS(s.hash + h, kSymEmpty, key) != kSymEmpty) h = (h + 1) & mask;
+  }
+  if (!barrier()) return kSymFailed;
+  auto find = [&](unsigned long long key) -> unsigned {      // its slot, or ~0 when not listed
+    unsigned h = sym_slot(key) & mask;
+    for (;;) {
+      const unsigned long long k = __ldcg(s.hash + h);
+      if (k == key) return h;
+      if (k == kSymEmpty) return ~0u;
+      h = (h + 1) & mask;
+    }
+  };
+  unsigned now = n;
+  for (int p = 0;; ++p) {
+    // a pair's level is stored as p + 1
+    late += 2ull * now;
+    unsigned rest = 0;
+    for (unsigned i = tid; i < n; i += nt) {
+      const unsigned long long e = __ldcg(s.list + i);
+      const unsigned v = (unsigned)(e >> 32), src = (unsigned)e;
+      const unsigned h = find(key_of_pair(v, src));
+      if (__ldcg(s.hlev + h) != 255) continue;
+      bool reached = false;
+      for (int j = 0; j < d && !reached; ++j) {
+        const unsigned u = (unsigned)__ldg(adj + (size_t)v * d + j);
+        const unsigned f = find(key_of_pair(u, src));
+        reached = f == ~0u || __ldcg(s.hlev + f) <= p;
+      }
+      if (reached) __stcg(s.hlev + h, (unsigned char)(p + 1));
+      else ++rest;
+    }
+    rest = __reduce_add_sync(0xffffffffu, rest);
+    if ((threadIdx.x & 31) == 0 && rest) atomicAdd(left + p, rest);
+    if (!barrier()) return kSymFailed;
+    const unsigned was = now;
+    now = __ldcg(left + p);
+    passes = p + 1;
+    if (now == 0) return kSymResolved;
+    if (now == was) return kSymStalled;
+    if (p + 1 == max_passes) return kSymTooLong;
   }
 }
 
@@ -557,66 +628,16 @@ __global__ void __launch_bounds__(kThreads, 1) apsp_sym_kernel(const ApspArgs a,
   }
   // ---- the listed pairs, level by level --------------------------------------------
   const unsigned n = stalled || fallback ? 0u : __ldcg(s.list_n);
-  unsigned long long late = 0;                 // sum of the unreached pairs at the levels after k*
+  unsigned long long late = 0;                 // sum of the unreached pairs at the levels from k* on
   int diam = last;
   if (n) {
-    unsigned size = 1024;
-    while (size < 2 * n) size <<= 1;
-    const unsigned mask = size - 1;
-    const unsigned tid = blockIdx.x * kThreads + threadIdx.x, nt = grid * kThreads;
-    for (unsigned i = tid; i < size; i += nt) {
-      __stcg(s.hash + i, kSymEmpty);
-      s.hlev[i] = 255;
-    }
-    if (!barrier()) return;
-    auto key_of_pair = [](unsigned x, unsigned y) {
-      return x > y ? ((unsigned long long)x << 32) | y : ((unsigned long long)y << 32) | x;
-    };
-    for (unsigned i = tid; i < n; i += nt) {
-      const unsigned long long e = __ldcg(s.list + i);
-      const unsigned long long key = key_of_pair((unsigned)(e >> 32), (unsigned)e);
-      unsigned h = sym_slot(key) & mask;
-      while (atomicCAS(s.hash + h, kSymEmpty, key) != kSymEmpty) h = (h + 1) & mask;
-    }
-    if (!barrier()) return;
-    auto find = [&](unsigned long long key) -> unsigned {      // its slot, or ~0 when not listed
-      unsigned h = sym_slot(key) & mask;
-      for (;;) {
-        const unsigned long long k = __ldcg(s.hash + h);
-        if (k == key) return h;
-        if (k == kSymEmpty) return ~0u;
-        h = (h + 1) & mask;
-      }
-    };
-    unsigned left = n;
-    for (int p = 0;; ++p) {
-      // pass p makes level k* + 1 + p; a pair's level is stored as p + 1
-      late += 2ull * left;
-      unsigned rest = 0;
-      for (unsigned i = tid; i < n; i += nt) {
-        const unsigned long long e = __ldcg(s.list + i);
-        const unsigned v = (unsigned)(e >> 32), src = (unsigned)e;
-        const unsigned h = find(key_of_pair(v, src));
-        if (__ldcg(s.hlev + h) != 255) continue;
-        bool reached = false;
-        for (int j = 0; j < d && !reached; ++j) {
-          const unsigned u = (unsigned)__ldg(a.adj + (size_t)v * d + j);
-          const unsigned f = find(key_of_pair(u, src));
-          reached = f == ~0u || __ldcg(s.hlev + f) <= p;
-        }
-        if (reached) __stcg(s.hlev + h, (unsigned char)(p + 1));
-        else ++rest;
-      }
-      rest = __reduce_add_sync(0xffffffffu, rest);
-      if ((threadIdx.x & 31) == 0 && rest) atomicAdd(s.list_n + 1 + p, rest);
-      if (!barrier()) return;
-      const unsigned now = __ldcg(s.list_n + 1 + p);
-      diam = last + 1 + p;
-      if (now == 0) break;
-      if (now == left) { stalled = true; break; }
-      if (p + 1 == kSymPasses) { fallback = true; break; }
-      left = now;
-    }
+    int passes = 0;
+    const int r = sym_resolve(s, s.list_n + 1, a.adj, d, n, kSymPasses, blockIdx.x * kThreads + threadIdx.x,
+                              grid * kThreads, barrier, late, passes);
+    if (r == kSymFailed) return;
+    diam = last + passes;
+    stalled = r == kSymStalled;
+    fallback = r == kSymTooLong;
   }
   if (fallback) {   // the persistent kernel launched behind this one runs instead
     if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->fallback = 1;
