@@ -1,20 +1,24 @@
 // apsp_batch.cu -- exact APSP of many graphs, of uneven sizes, in one launch.
 //
 // A batch is a fixed list of graphs (nodes, based_nodes, groups, degree each)
-// whose adjacency arrays sit packed in one device buffer.  One cooperative
-// launch of apsp_batch_kernel evaluates all of them: the launch's CTAs form
-// teams of `team_ctas` CTAs, the graphs are dealt to the teams longest-first
-// (each to the team with the least modelled work so far), and every team
-// runs its graphs' source windows exactly as the single-graph kernel runs one
-// graph's, with a barrier of its own.  Per graph the answer is the one
-// ggb_eval_general gives (general/evaluation.c:153-263 per graph); the plan
-// -- window width and team size -- changes only the time.
+// whose adjacency arrays sit packed in one device buffer.  A fixed plan
+// evaluates all of them in one cooperative launch of apsp_batch_kernel: the
+// launch's CTAs form teams of `team_ctas` CTAs, the graphs are dealt to the
+// teams longest-first (each to the team with the least modelled work so far),
+// and every team runs its graphs' source windows exactly as the single-graph
+// kernel runs one graph's, with a barrier of its own.  The automatic plan
+// (plan_split) sends small graphs to shared-memory windows and mid-size ones to
+// level-by-level teams first, each in launches of their own.  Per graph the
+// answer is the one ggb_eval_general gives (general/evaluation.c:153-263 per
+// graph); the plan changes only the time.
 //
-// The launch (two memsets of the control blocks and the kernel) is captured
-// once per plan in a CUDA graph and replayed, so a step of a batched
-// annealing loop costs one graph launch.  ggb_batch_autotune times every
-// feasible (window width, team size) pair on the batch's current adjacency
-// and keeps the fastest.
+// The launches (with the memsets of their control blocks) are captured once per
+// plan in a CUDA graph and replayed, so a step of a batched annealing loop costs
+// one graph launch.  ggb_batch_autotune times the automatic plan and every
+// feasible (window width, team size) pair on the batch's current adjacency and
+// keeps the fastest.  The mixed workload of 257 graphs (512 to 16384 vertices,
+// d = 12): 4.6 ms of kernels with the automatic plan, 5.7 ms with the best fixed
+// one.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -29,6 +33,8 @@
 
 #include "../../include/graphgolf_b200.h"
 #include "apsp_kernel.cuh"
+#include "apsp_levels.cuh"
+#include "apsp_slice.cuh"
 #include "batch_internal.h"
 #include "core_internal.h"
 
@@ -90,6 +96,17 @@ int dev_alloc(T** p, size_t n) {
 
 namespace {
 
+template <typename T>
+int regrow(T** p, size_t* cap, size_t n) {
+  if (n <= *cap && *p) return GGB_OK;
+  cudaFree(*p);
+  *p = nullptr;
+  *cap = 0;
+  const int rc = dev_alloc(p, n);
+  if (rc == GGB_OK) *cap = n;
+  return rc;
+}
+
 // Modelled seconds of one graph on a team of T CTAs with windows of 128*R
 // sources: per window the two-hop seeding plus about five dense sweeps of
 // d gathered 16R-byte rows per vertex, each sweep at least one memory round
@@ -108,14 +125,13 @@ double graph_cost(int N, int d, int nsrc, int R, int T) {
 // Deals the graphs to the teams (longest first, each to the least loaded
 // team) and returns the modelled makespan; fills the plan arrays when
 // `keep`.
-double make_plan(ggb_batch* b, int R, int T, bool keep) {
+double make_plan(ggb_batch* b, const std::vector<int>& ids, int R, int T, bool keep) {
   const int ctas_max = b->occ[log2i(R)] * b->sms;
   T = std::max(1, std::min(T, ctas_max));
-  int n_teams = std::max(1, std::min(ctas_max / T, b->n));
+  int n_teams = std::max(1, std::min(ctas_max / T, (int)ids.size()));
   std::vector<double> cost(b->n);
-  for (int i = 0; i < b->n; ++i) cost[i] = graph_cost(b->N[i], b->d[i], b->bn[i], R, T);
-  std::vector<int> order(b->n);
-  std::iota(order.begin(), order.end(), 0);
+  for (int i : ids) cost[i] = graph_cost(b->N[i], b->d[i], b->bn[i], R, T);
+  std::vector<int> order(ids);
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
   using Load = std::pair<double, int>;
   std::priority_queue<Load, std::vector<Load>, std::greater<Load>> pq;
@@ -131,14 +147,16 @@ double make_plan(ggb_batch* b, int R, int T, bool keep) {
     pq.push(l);
   }
   // Working set of the teams running at once: each team's adjacency and two
-  // matrices.  Past about 60% of L2 the gathers spill to HBM.
+  // matrices.  Past the L2 size the gathers spill to HBM, at a mild price (51
+  // graphs of 8192 to 16384 vertices, R = 32: 3.8 ms on 6 teams of 24 CTAs,
+  // 100 MB, 4.4 ms on 18 of 8, 315 MB).
   double ws = 0.0;
   for (int t = 0; t < n_teams; ++t) {
     long long mx = 0;
     for (int i : lists[t]) mx = std::max<long long>(mx, (long long)b->N[i] * (b->d[i] * 4 + 32 * R));
     ws += (double)mx;
   }
-  if (ws > 0.6 * (double)b->l2) makespan *= 1.0 + 1.5 * std::min(1.0, (ws - 0.6 * b->l2) / (0.6 * b->l2));
+  if (ws > (double)b->l2) makespan *= 1.0 + 0.12 * (ws / (double)b->l2 - 1.0);
   if (!keep) return makespan;
   b->R = R;
   b->T = T;
@@ -165,7 +183,7 @@ double make_plan(ggb_batch* b, int R, int T, bool keep) {
   b->team_soff.assign(n_teams, 0);
   b->stamp_ints = 0;
   bool stamping = false;
-  for (int i = 0; i < b->n; ++i) stamping = stamping || (R == 32 && b->d[i] <= 16);
+  for (int i : ids) stamping = stamping || (R == 32 && b->d[i] <= 16);
   if (stamping) {
     for (int t = 0; t < n_teams; ++t) {
       int mx = 0;
@@ -185,18 +203,10 @@ int drop_graph(ggb_batch* b) {
   return GGB_OK;
 }
 
-// Uploads the plan made by make_plan(keep = true).
-int upload_plan(ggb_batch* b) {
-  drop_graph(b);
-  const long long cells = b->team_off.back() + 2 * b->team_cells.back();
-  if ((size_t)cells > b->cap_scratch) {
-    if (b->d_scratch) cudaFree(b->d_scratch);
-    b->d_scratch = nullptr;
-    b->cap_scratch = 0;
-    int rc = dev_alloc(&b->d_scratch, (size_t)cells);
-    if (rc) return rc;
-    b->cap_scratch = (size_t)cells;
-  }
+// Uploads the windows plan made by make_plan(keep = true).
+int upload_windows(ggb_batch* b) {
+  if (int rc = regrow(&b->d_scratch, &b->cap_scratch, (size_t)(b->team_off.back() + 2 * b->team_cells.back())))
+    return rc;
   BCUDA(cudaMemcpyAsync(b->d_tstart, b->team_start.data(), b->team_start.size() * sizeof(int),
                         cudaMemcpyHostToDevice, b->stream));
   BCUDA(cudaMemcpyAsync(b->d_tlist, b->team_list.data(), b->team_list.size() * sizeof(int),
@@ -221,6 +231,189 @@ int upload_plan(ggb_batch* b) {
   return GGB_OK;
 }
 
+// ---- the automatic plan ----------------------------------------------------------
+
+constexpr size_t kSliceSmemMax = 224 * 1024;
+
+std::vector<int> all_graphs(const ggb_batch* b) {
+  std::vector<int> ids(b->n);
+  std::iota(ids.begin(), ids.end(), 0);
+  return ids;
+}
+
+// Modelled seconds of one graph level by level on T CTAs (measured at
+// N = 16384, d = 12: 11 ms / T + 70 us).
+double levels_cost(int N, int d, int T) {
+  const double x = N / 16384.0;
+  return 11.0e-3 * x * x * (d + 1) / 13.0 / T + 70.0e-6;
+}
+
+// Slices for the graphs of `ids`: rows of 32 sources while every window then
+// has an SM to itself (one step of an annealer), else of 64 (fewer stagings and
+// fewer wavefronts a source).  Launches by shared memory, largest graphs first.
+void plan_slices(ggb_batch* b, const std::vector<int>& ids) {
+  b->slices.clear();
+  b->slice_items.clear();
+  long long w32 = 0;
+  for (int i : ids) w32 += (b->bn[i] + 31) / 32;
+  const int words = w32 <= b->sms ? 1 : 2, width = 32 * words;
+  long long windows = 0;
+  for (int i : ids) windows += (b->bn[i] + width - 1) / width;
+  const int per = (int)std::max<long long>(1, windows / (8LL * b->sms));   // windows a CTA
+  auto smem = [&](int i) { return ggb::slice_smem_bytes((b->N[i] + 31) / 32 * 32, words, (b->d[i] + 1) / 2); };
+  std::vector<int> order(ids);
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return smem(x) > smem(y); });
+  const size_t limit[3] = {72 * 1024, 110 * 1024, kSliceSmemMax};   // three, two CTAs or one an SM
+  int bucket = -1;
+  for (int i : order) {
+    const size_t sm = smem(i);
+    const int k = sm <= limit[0] ? 0 : sm <= limit[1] ? 1 : 2;
+    if (k != bucket) {
+      b->slices.push_back({words, 0, (int)b->slice_items.size(), 0, sm});
+      bucket = k;
+    }
+    auto& launch = b->slices.back();
+    const int np = (b->N[i] + 31) / 32 * 32;
+    launch.threads = std::max(launch.threads, std::min(np, k == 0 ? 640 : k == 1 ? 768 : 1024));
+    const int nw = (b->bn[i] + width - 1) / width, ctas = (nw + per - 1) / per;
+    for (int t = 0; t < nw; t += per) b->slice_items.push_back({i, t, std::min(nw, t + per), ctas});
+    launch.items = (int)b->slice_items.size() - launch.first;
+    b->slice_words[i] = words;
+  }
+}
+
+// Level-by-level teams for the graphs of `ids`: the team size with the least
+// modelled makespan.
+void plan_levels(ggb_batch* b, const std::vector<int>& ids) {
+  b->l_teams = 0;
+  if (ids.empty()) return;
+  double best = 1e300;
+  for (int T : {148, 74, 49, 37, 29, 24, 21, 18, 16}) {
+    T = std::min(T, b->sms);
+    const int n_teams = std::max(1, std::min(b->sms / T, (int)ids.size()));
+    std::vector<int> order(ids);
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+      return levels_cost(b->N[x], b->d[x], T) > levels_cost(b->N[y], b->d[y], T);
+    });
+    std::vector<double> load(n_teams, 0.0);
+    std::vector<std::vector<int>> lists(n_teams);
+    for (int i : order) {
+      const int t = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+      load[t] += levels_cost(b->N[i], b->d[i], T);
+      lists[t].push_back(i);
+    }
+    const double m = *std::max_element(load.begin(), load.end());
+    if (m >= best * 0.999) continue;
+    best = m;
+    b->lT = T;
+    b->l_teams = n_teams;
+    b->l_start.assign(1, 0);
+    b->l_list.clear();
+    b->l_off.clear();
+    b->l_cells.clear();
+    b->l_smem = 0;
+    long long off = 0;
+    for (const auto& l : lists) {
+      long long cells = 0;
+      for (int i : l) {
+        b->l_list.push_back(i);
+        cells = std::max<long long>(cells, (long long)b->N[i] * ggb::levels_pitch(b->N[i]));
+        b->l_smem = std::max(b->l_smem, ggb::levels_smem_bytes(b->N[i], b->d[i]));
+      }
+      b->l_start.push_back((int)b->l_list.size());
+      b->l_off.push_back(off);
+      b->l_cells.push_back(cells);
+      off += 2 * cells;
+    }
+  }
+}
+
+int upload_split(ggb_batch* b) {
+  int rc;
+  if (!b->slice_items.empty()) {
+    if ((rc = regrow(&b->d_items, &b->cap_items, b->slice_items.size()))) return rc;
+    BCUDA(cudaMemcpyAsync(b->d_items, b->slice_items.data(), b->slice_items.size() * sizeof(ggb::SliceItem),
+                          cudaMemcpyHostToDevice, b->stream));
+  }
+  if (b->l_teams > 0) {
+    const size_t nt = (size_t)b->l_teams;
+    const size_t words = ggb::kLevelsListWords + (ggb::kLevelsCounters + 1) / 2;
+    if ((rc = regrow(&b->d_lint, &b->cap_lint, nt + 1 + b->l_list.size())) ||
+        (rc = regrow(&b->d_lll, &b->cap_lll, 2 * nt)) || (rc = regrow(&b->d_lists, &b->cap_lists, nt * words)) ||
+        (rc = regrow(&b->d_scratch, &b->cap_scratch, (size_t)(b->l_off.back() + 2 * b->l_cells.back()))))
+      return rc;
+    BCUDA(cudaMemcpyAsync(b->d_lint, b->l_start.data(), (nt + 1) * sizeof(int), cudaMemcpyHostToDevice, b->stream));
+    BCUDA(cudaMemcpyAsync(b->d_lint + nt + 1, b->l_list.data(), b->l_list.size() * sizeof(int),
+                          cudaMemcpyHostToDevice, b->stream));
+    BCUDA(cudaMemcpyAsync(b->d_lll, b->l_off.data(), nt * sizeof(long long), cudaMemcpyHostToDevice, b->stream));
+    BCUDA(cudaMemcpyAsync(b->d_lll + nt, b->l_cells.data(), nt * sizeof(long long), cudaMemcpyHostToDevice,
+                          b->stream));
+  }
+  BCUDA(cudaStreamSynchronize(b->stream));
+  return GGB_OK;
+}
+
+void model_choice(ggb_batch* b, const std::vector<int>& ids, int* R, int* T);
+
+// The automatic plan.  Falls back to one windows plan for all graphs when the
+// level-by-level workspace cannot be had.
+int plan_split(ggb_batch* b) {
+  drop_graph(b);
+  b->split = true;
+  b->slice_words.assign(b->n, 0);
+  // Slices: as for a single graph (plan_slice in apsp_core.cu) while every
+  // window has an SM to itself; with more windows than that they only pay for
+  // smaller graphs (102 graphs of 512 to 3460 vertices, d = 12: 401 us, 393 on
+  // teams; 65 of 256 to 4096, d = 8: 162 / 219; 64 of 1024, d = 8: 52 / 61).
+  // Level by level: from 8193 vertices like a single graph; with teams enough
+  // to hide its barriers from 4500 (52 graphs of 4096 to 8192 vertices, d = 12:
+  // 1198 us, 1309 from 6000 on, 1462 as windows).
+  long long w32 = 0;
+  int over = 0;
+  for (int i = 0; i < b->n; ++i) {
+    w32 += (b->bn[i] + 31) / 32;
+    over += b->N[i] > 4500;
+  }
+  const long long most = w32 <= b->sms ? 45000 : 30000;
+  const int from = over >= 8 ? 4500 : 8192;
+  std::vector<int> small, mid, rest;
+  for (int i = 0; i < b->n; ++i) {
+    const int N = b->N[i], d = b->d[i];
+    const size_t smem = ggb::slice_smem_bytes((N + 31) / 32 * 32, 2, (d + 1) / 2);
+    if ((long long)N * (d + 1) <= most && N <= ggb::kSliceMaxN && smem <= kSliceSmemMax) small.push_back(i);
+    else if (b->grp[i] == 1 && d >= 4 && d <= 32 && N > from && N <= 22000) mid.push_back(i);
+    else rest.push_back(i);
+  }
+  plan_slices(b, small);
+  plan_levels(b, mid);
+  int rc = upload_split(b);
+  if (rc == GGB_ENOMEM) {
+    b->l_teams = 0;
+    rest.insert(rest.end(), mid.begin(), mid.end());
+    rc = GGB_OK;
+  }
+  if (rc) return rc;
+  b->n_teams = b->ctas = 0;
+  b->stamp_ints = 0;
+  if (rest.empty()) return GGB_OK;
+  int R = 1, T = 1;
+  model_choice(b, rest, &R, &T);
+  make_plan(b, rest, R, T, true);
+  return upload_windows(b);
+}
+
+// One windows plan for all graphs.
+int plan_fixed(ggb_batch* b, int R, int T) {
+  drop_graph(b);
+  b->split = false;
+  b->slices.clear();
+  b->slice_items.clear();
+  b->slice_words.assign(b->n, 0);
+  b->l_teams = 0;
+  make_plan(b, all_graphs(b), R, T, true);
+  return upload_windows(b);
+}
+
 ggb::BatchArgs batch_args(const ggb_batch* b) {
   ggb::BatchArgs a;
   a.graphs = b->d_graphs;
@@ -243,24 +436,72 @@ ggb::BatchArgs batch_args(const ggb_batch* b) {
 
 }  // namespace
 
-// The launch itself: zero the control blocks and results, then the kernel.
-int ggb::batch_enqueue(ggb_batch* b, cudaStream_t st) {
-  BCUDA(cudaMemsetAsync(b->d_ctrl, 0, (size_t)b->n_teams * sizeof(ggb::ApspCtrl), st));
-  BCUDA(cudaMemsetAsync(b->d_out, 0, (size_t)b->n * sizeof(ggb::BatchOut), st));
-  if (b->stamp_ints > 0) BCUDA(cudaMemsetAsync(b->d_stamps, 0, (size_t)b->stamp_ints * sizeof(unsigned), st));
-  ggb::BatchArgs args = batch_args(b);
+namespace {
+
+int coop(const void* fn, int ctas, size_t smem, void** params, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(b->ctas);
+  cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(ggb::kThreads);
-  cfg.dynamicSmemBytes = batch_smem_for(b->R);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  void* params[] = {(void*)&args};
-  BCUDA(cudaLaunchKernelExC(&cfg, batch_kernel_for(b->R), params));
+  BCUDA(cudaLaunchKernelExC(&cfg, fn, params));
+  return GGB_OK;
+}
+
+}  // namespace
+
+// The launches themselves: the largest work first.  The slices clear nothing
+// and need nothing cleared; the teams' control blocks and results are zeroed.
+int ggb::batch_enqueue(ggb_batch* b, cudaStream_t st) {
+  int rc;
+  if (b->l_teams > 0 || b->n_teams > 0)
+    BCUDA(cudaMemsetAsync(b->d_out, 0, (size_t)b->n * sizeof(ggb::BatchOut), st));
+  if (b->l_teams > 0) {
+    const size_t words = ggb::kLevelsListWords + (ggb::kLevelsCounters + 1) / 2;
+    BCUDA(cudaMemsetAsync(b->d_lctrl, 0, (size_t)2 * b->l_teams * sizeof(ggb::ApspCtrl), st));
+    BCUDA(cudaMemset2DAsync(b->d_lists + ggb::kLevelsListWords, words * 8, 0, ggb::kLevelsCounters * sizeof(unsigned),
+                            b->l_teams, st));
+    ggb::BatchArgs a = batch_args(b);
+    a.team_ctrl = b->d_lctrl;
+    a.team_start = b->d_lint;
+    a.team_list = b->d_lint + b->l_teams + 1;
+    a.scratch = b->d_scratch;   // the launches of a batch follow one another: one scratch
+    a.team_off = b->d_lll;
+    a.team_cells = b->d_lll + b->l_teams;
+    a.n_teams = b->l_teams;
+    a.team_ctas = b->lT;
+    a.stamps = nullptr;
+    a.team_soff = nullptr;
+    size_t w = words;
+    void* params[] = {(void*)&a, (void*)&b->d_lists, (void*)&w};
+    if ((rc = coop((const void*)ggb::apsp_batch_levels_kernel, b->l_teams * b->lT, b->l_smem, params, st))) return rc;
+    // graphs that were not served: asymmetric ones, or with too many levels past the list
+    a.behind = b->d_lctrl;
+    a.team_ctrl = b->d_lctrl + b->l_teams;
+    void* params2[] = {(void*)&a};
+    if ((rc = coop(batch_kernel_for(32), b->l_teams * b->lT, batch_smem_for(32), params2, st))) return rc;
+  }
+  if (b->n_teams > 0) {
+    BCUDA(cudaMemsetAsync(b->d_ctrl, 0, (size_t)b->n_teams * sizeof(ggb::ApspCtrl), st));
+    if (b->stamp_ints > 0) BCUDA(cudaMemsetAsync(b->d_stamps, 0, (size_t)b->stamp_ints * sizeof(unsigned), st));
+    ggb::BatchArgs args = batch_args(b);
+    void* params[] = {(void*)&args};
+    if ((rc = coop(batch_kernel_for(b->R), b->ctas, batch_smem_for(b->R), params, st))) return rc;
+  }
+  for (const auto& l : b->slices) {
+    if (l.words == 1)
+      ggb::slice_batch_kernel<1><<<l.items, l.threads, l.smem, st>>>(b->d_graphs, b->d_items + l.first, b->d_records,
+                                                                    b->d_out, b->stop, b->sticky);
+    else
+      ggb::slice_batch_kernel<2><<<l.items, l.threads, l.smem, st>>>(b->d_graphs, b->d_items + l.first, b->d_records,
+                                                                    b->d_out, b->stop, b->sticky);
+    BCUDA(cudaGetLastError());
+  }
   return GGB_OK;
 }
 
@@ -302,24 +543,48 @@ int launch(ggb_batch* b, cudaStream_t st, bool use_graph) {
   return GGB_OK;
 }
 
+// Sources per window of graph i under the current plan.
+int window_bits_of(const ggb_batch* b, int i) {
+  if (!b->split) return 128 * b->R;
+  if (b->slice_words[i]) return 32 * b->slice_words[i];
+  if (b->l_teams > 0 && std::find(b->l_list.begin(), b->l_list.end(), i) != b->l_list.end())
+    return 128 * ggb::levels_pitch(b->N[i]);
+  return 128 * b->R;
+}
+
 int collect(ggb_batch* b, cudaStream_t st, ggb_result* res) {
   BCUDA(cudaMemcpyAsync(b->h_out, b->d_out, (size_t)b->n * sizeof(ggb::BatchOut), cudaMemcpyDeviceToHost, st));
-  BCUDA(cudaMemcpyAsync(b->h_ctrl, b->d_ctrl, (size_t)b->n_teams * sizeof(ggb::ApspCtrl), cudaMemcpyDeviceToHost,
-                        st));
+  if (b->n_teams > 0)
+    BCUDA(cudaMemcpyAsync(b->h_ctrl, b->d_ctrl, (size_t)b->n_teams * sizeof(ggb::ApspCtrl), cudaMemcpyDeviceToHost,
+                          st));
+  if (b->l_teams > 0)
+    BCUDA(cudaMemcpyAsync(b->h_lctrl, b->d_lctrl, (size_t)2 * b->l_teams * sizeof(ggb::ApspCtrl),
+                          cudaMemcpyDeviceToHost, st));
   BCUDA(cudaStreamSynchronize(st));
   b->pending = false;
-  for (int t = 0; t < b->n_teams; ++t) {
-    const ggb::ApspCtrl& c = b->h_ctrl[t];
-    if (c.error == 0) continue;
-    int gi = -1;
-    for (int k = b->team_start[t]; k < b->team_start[t + 1]; ++k)
-      if (!b->h_out[b->team_list[k]].done) { gi = b->team_list[k]; break; }
-    if (c.error == ggb::kErrAdj)
+  auto report = [&](int error, int info, int gi) {
+    if (error == ggb::kErrAdj)
       return core_fail(GGB_EADJ, "batch graph %d: adjacency entry outside [0, nodes)", gi);
-    if (c.error == ggb::kErrTimeout)
-      return core_fail(GGB_ETIMEOUT, "batch graph %d: a team-barrier wait ran out (CTA %d)", gi, c.error_info);
-    return core_fail(GGB_ECUDA, "batch graph %d: device error code %d", gi, c.error);
+    if (error == ggb::kErrTimeout)
+      return core_fail(GGB_ETIMEOUT, "batch graph %d: a team-barrier wait ran out (CTA %d)", gi, info);
+    return core_fail(GGB_ECUDA, "batch graph %d: device error code %d", gi, error);
+  };
+  // a team that failed left its graphs from the failing one on undone
+  auto check_team = [&](const ggb::ApspCtrl& c, const int* list, int k0, int k1) {
+    if (c.error == 0) return (int)GGB_OK;
+    for (int k = k0; k < k1; ++k)
+      if (!b->h_out[list[k]].done) return report(c.error, c.error_info, list[k]);
+    return report(c.error, c.error_info, -1);
+  };
+  int rc;
+  for (int t = 0; t < b->n_teams; ++t)
+    if ((rc = check_team(b->h_ctrl[t], b->team_list.data(), b->team_start[t], b->team_start[t + 1]))) return rc;
+  for (int t = 0; t < 2 * b->l_teams; ++t) {
+    const int k = t % b->l_teams;
+    if ((rc = check_team(b->h_lctrl[t], b->l_list.data(), b->l_start[k], b->l_start[k + 1]))) return rc;
   }
+  for (int i = 0; i < b->n; ++i)
+    if (b->h_out[i].error) return report(b->h_out[i].error, 0, i);
   for (int i = 0; i < b->n; ++i) {
     const ggb::BatchOut& o = b->h_out[i];
     if (!o.done) return core_fail(GGB_ECUDA, "batch graph %d was not evaluated", i);
@@ -330,9 +595,9 @@ int collect(ggb_batch* b, cudaStream_t st, ggb_result* res) {
     p.sum = o.sum;
     p.levels = o.levels;
     p.windows = o.windows;
-    p.window_bits = 128 * b->R;
+    p.window_bits = window_bits_of(b, i);
     p.dense_levels = o.dense_levels;
-    int rc = ggb_finish_general(b->N[i], &p, res + i);
+    rc = ggb_finish_general(b->N[i], &p, res + i);
     if (rc) return rc;
   }
   return GGB_OK;
@@ -358,6 +623,13 @@ void destroy(ggb_batch* b) {
   cudaFree(b->d_tsoff);
   cudaFree(b->d_stamps);
   cudaFree(b->d_scratch);
+  cudaFree(b->d_items);
+  cudaFree(b->d_records);
+  cudaFree(b->d_lint);
+  cudaFree(b->d_lll);
+  cudaFree(b->d_lctrl);
+  cudaFreeHost(b->h_lctrl);
+  cudaFree(b->d_lists);
   for (auto& e : b->ev)
     if (e) cudaEventDestroy(e);
   if (b->stream) cudaStreamDestroy(b->stream);
@@ -402,6 +674,9 @@ int create(int n_graphs, const int* nodes, const int* based_nodes, const int* gr
     b->occ[log2i(R)] = nb;
     b->max_teams = std::max(b->max_teams, nb * b->sms);
   }
+  for (const void* k : {(const void*)ggb::slice_batch_kernel<1>, (const void*)ggb::slice_batch_kernel<2>,
+                        (const void*)ggb::apsp_batch_levels_kernel})
+    BCUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSliceSmemMax));
   if (const char* s = getenv("GGB_BARRIER_TIMEOUT_NS")) b->timeout_ns = atoll(s);
   BCUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
   BCUDA(cudaEventCreate(&b->ev[0]));
@@ -427,6 +702,9 @@ int create(int n_graphs, const int* nodes, const int* based_nodes, const int* gr
   if ((rc = dev_alloc(&b->d_toff, mt))) return rc;
   if ((rc = dev_alloc(&b->d_tcells, mt))) return rc;
   if ((rc = dev_alloc(&b->d_tsoff, mt))) return rc;
+  if ((rc = dev_alloc(&b->d_records, (size_t)n_graphs)) || (rc = dev_alloc(&b->d_lctrl, 2 * mt))) return rc;
+  BCUDA(cudaMemset(b->d_records, 0, (size_t)n_graphs * sizeof(ggb::ApspCtrl)));
+  BCUDA(cudaHostAlloc(&b->h_lctrl, 2 * mt * sizeof(ggb::ApspCtrl), cudaHostAllocDefault));
   BCUDA(cudaHostAlloc(&b->h_out, (size_t)n_graphs * sizeof(ggb::BatchOut), cudaHostAllocDefault));
   BCUDA(cudaHostAlloc(&b->h_ctrl, mt * sizeof(ggb::ApspCtrl), cudaHostAllocDefault));
   std::vector<ggb::BatchGraph> gs(n_graphs);
@@ -447,12 +725,14 @@ int create(int n_graphs, const int* nodes, const int* based_nodes, const int* gr
 }
 
 // The plan the model prefers: the (R, T) pair with the least modelled makespan.
-void model_choice(ggb_batch* b, int* R, int* T) {
+void model_choice(ggb_batch* b, const std::vector<int>& ids, int* R, int* T) {
   double best = 1e300;
-  int nsrc_max = *std::max_element(b->bn.begin(), b->bn.end());
+  int nsrc_max = 0;
+  for (int i : ids) nsrc_max = std::max(nsrc_max, b->bn[i]);
   for (int r = 1; r <= kMaxR; r *= 2) {
-    for (int t = 1; t <= b->occ[log2i(r)] * b->sms; t *= 2) {
-      const double m = make_plan(b, r, t, false);
+    for (int t : {1, 2, 4, 8, 16, 24, 37, 49, 74, 148}) {
+      if (t > b->occ[log2i(r)] * b->sms) break;
+      const double m = make_plan(b, ids, r, t, false);
       if (m < best * 0.999) { best = m; *R = r; *T = t; }
     }
     if (128 * r >= nsrc_max) break;
@@ -487,21 +767,23 @@ int ggb_batch_set_plan(ggb_batch* b, int window_bits, int team_ctas) {
   if (window_bits && (window_bits % 128 || (R & (R - 1)) || R > kMaxR))
     return core_fail(GGB_EINVAL, "window_bits must be 128 * 2^k, at most %d", 128 * kMaxR);
   BCUDA(cudaSetDevice(b->device));
+  if (!R && !T) return plan_split(b);
   if (!R || !T) {
     int mr = 1, mt = 1;
-    model_choice(b, &mr, &mt);
+    model_choice(b, all_graphs(b), &mr, &mt);
     if (!R) R = mr;
     if (!T) T = mt;
   }
-  make_plan(b, R, T, true);
-  return upload_plan(b);
+  return plan_fixed(b, R, T);
 }
 
 int ggb_batch_get_plan(const ggb_batch* b, int* window_bits, int* team_ctas, int* teams) {
   if (!b) return core_fail(GGB_EINVAL, "null batch");
-  if (window_bits) *window_bits = 128 * b->R;
-  if (team_ctas) *team_ctas = b->T;
-  if (teams) *teams = b->n_teams;
+  // the automatic plan: its windows teams, else its level-by-level teams, else its slices
+  const bool win = b->n_teams > 0, lev = !win && b->l_teams > 0;
+  if (window_bits) *window_bits = win ? 128 * b->R : lev ? 4096 : 128;
+  if (team_ctas) *team_ctas = win ? b->T : lev ? b->lT : 1;
+  if (teams) *teams = win ? b->n_teams : lev ? b->l_teams : (int)b->slice_items.size();
   return GGB_OK;
 }
 
@@ -563,7 +845,21 @@ int ggb_batch_autotune(ggb_batch* b, int iters, int* window_bits, int* team_ctas
   BCUDA(cudaSetDevice(b->device));
   const int nsrc_max = *std::max_element(b->bn.begin(), b->bn.end());
   double best = 1e300;
-  int bR = b->R, bT = b->T;
+  int bR = 0, bT = 0, rc;
+  // the least time of `iters` launches of the current plan, after one that warms up
+  auto time_plan = [&](double* ms_min) -> int {
+    *ms_min = 1e300;
+    for (int it = 0; it <= iters; ++it) {
+      int rc = launch(b, b->stream, false);
+      if (rc) return rc;
+      if ((rc = collect(b, b->stream, nullptr))) return rc;
+      float f = 0.f;
+      BCUDA(cudaEventElapsedTime(&f, b->ev[0], b->ev[1]));
+      if (it > 0) *ms_min = std::min(*ms_min, (double)f);
+    }
+    return GGB_OK;
+  };
+  if ((rc = plan_split(b)) || (rc = time_plan(&best))) return rc;   // bR == 0: the automatic plan
   for (int r = 1; r <= kMaxR; r *= 2) {
     const int ctas_max = b->occ[log2i(r)] * b->sms;
     std::vector<int> ts;
@@ -571,28 +867,15 @@ int ggb_batch_autotune(ggb_batch* b, int iters, int* window_bits, int* team_ctas
     for (int t : {b->sms / 4, b->sms / 2, b->sms})
       if (t >= 1 && t <= ctas_max && std::find(ts.begin(), ts.end(), t) == ts.end()) ts.push_back(t);
     for (int t : ts) {
-      make_plan(b, r, t, true);
-      int rc = upload_plan(b);
-      if (rc) return rc;
-      double ms_min = 1e300;
-      for (int it = 0; it <= iters; ++it) {
-        rc = launch(b, b->stream, false);
-        if (rc) return rc;
-        rc = collect(b, b->stream, nullptr);
-        if (rc) return rc;
-        float f = 0.f;
-        BCUDA(cudaEventElapsedTime(&f, b->ev[0], b->ev[1]));
-        if (it > 0) ms_min = std::min(ms_min, (double)f);   // the first launch warms up
-      }
-      if (ms_min < best) { best = ms_min; bR = r; bT = t; }
+      double ms = 0.0;
+      if ((rc = plan_fixed(b, r, t)) || (rc = time_plan(&ms))) return rc;
+      if (ms < best) { best = ms; bR = r; bT = t; }
     }
     if (128 * r >= nsrc_max) break;   // wider windows only add zero bits
   }
-  make_plan(b, bR, bT, true);
-  int rc = upload_plan(b);
+  rc = bR ? plan_fixed(b, bR, bT) : plan_split(b);
   if (rc) return rc;
-  if (window_bits) *window_bits = 128 * bR;
-  if (team_ctas) *team_ctas = bT;
+  if ((rc = ggb_batch_get_plan(b, window_bits, team_ctas, nullptr))) return rc;
   if (best_ms) *best_ms = best;
   return GGB_OK;
 }

@@ -815,6 +815,8 @@ __global__ void delta_reduce_kernel(const DeltaArgs a, const BaseResult* __restr
     r.diam = stalled ? a.N + 1 : mx;
     r.disconnected = stalled;
     r.windows = a.nwin;
+    r.error = 0;
+    r.pad_ = 0;
     r.done = (missing || base->disconnected) ? 0 : 1;
     out[c] = r;
   }

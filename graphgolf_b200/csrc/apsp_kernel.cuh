@@ -1364,9 +1364,16 @@ struct BatchGraph {
   int win_bits;          // sources per window below 128 * R (64), or 0
 };
 
+// One CTA of a launch of many small graphs (apsp_slice.cuh).
+struct SliceItem {
+  int graph, first, end;   // windows first .. end - 1
+  int ctas;                // CTAs of the graph
+};
+
 struct BatchOut {        // per graph, written by the team's first CTA
   long long sum, levels, dense_levels;
   int diam, disconnected, windows, done;
+  int error, pad_;       // first error of a graph without a team (slices), else 0
 };
 
 struct BatchArgs {
@@ -1386,6 +1393,10 @@ struct BatchArgs {
   // stamps + team_soff[t], one per vertex of its largest graph.
   unsigned* stamps = nullptr;
   const long long* team_soff = nullptr;
+  // When given, the launch takes only the graphs that the level-by-level
+  // launch before it left (out[].done == 0), and nothing when a team of it
+  // failed.
+  const ApspCtrl* behind = nullptr;
 };
 
 template <int R>
@@ -1396,6 +1407,7 @@ __global__ void __launch_bounds__(kThreads, 1) apsp_batch_kernel(const BatchArgs
   const int cta = (int)blockIdx.x % b.team_ctas;
   if (team >= b.n_teams) return;
   if (b.stop && ld_volatile_i32(b.stop) != 0) return;   // written before the launch: the same in every CTA
+  if (b.behind && ld_volatile_i32(&b.behind[team].error) != 0) return;
   if (threadIdx.x < 8) sm.seen[threadIdx.x >> 1][threadIdx.x & 1] = 0ULL;
   __syncthreads();
   ApspArgs a;
@@ -1423,6 +1435,7 @@ __global__ void __launch_bounds__(kThreads, 1) apsp_batch_kernel(const BatchArgs
   const int k1 = b.team_start[team + 1];
   for (int k = b.team_start[team]; k < k1; ++k) {
     const int gi = b.team_list[k];
+    if (b.behind && ld_volatile_i32(&b.out[gi].done) != 0) continue;   // this launch writes it after the team's last read
     const BatchGraph gr = b.graphs[gi];
     a.adj = gr.adj;
     a.N = gr.N;
@@ -1447,6 +1460,7 @@ __global__ void __launch_bounds__(kThreads, 1) apsp_batch_kernel(const BatchArgs
       w->diam = o.diam;
       w->disconnected = o.disconnected;
       w->windows = o.windows;
+      w->error = 0;
       w->done = 1;
     }
     // the next graph's windows take the stamp ids after this graph's

@@ -331,7 +331,7 @@ __device__ __forceinline__ int eval_levels(const ApspArgs& a, const LevelsList& 
 }
 
 // ---- one graph, one team ---------------------------------------------------------
-__global__ void __launch_bounds__(kThreads, 1) apsp_levels_kernel(const ApspArgs a, const LevelsList ws) {
+static __global__ void __launch_bounds__(kThreads, 1) apsp_levels_kernel(const ApspArgs a, const LevelsList ws) {
   __shared__ ApspSmem sm;
   extern __shared__ __align__(16) unsigned s_dyn[];
   if (threadIdx.x < 8) sm.seen[threadIdx.x >> 1][threadIdx.x & 1] = 0ULL;
@@ -354,6 +354,61 @@ __global__ void __launch_bounds__(kThreads, 1) apsp_levels_kernel(const ApspArgs
   c->windows = o.windows;
   __threadfence();
   c->done = 1;
+}
+
+// ---- many graphs on teams, as apsp_batch_kernel --------------------------------------
+// b.scratch + b.team_off[t] holds team t's two matrices (b.team_cells[t] apart),
+// lists + t * list_words its list.  A graph that is not served keeps done = 0
+// for the window launch behind this one.
+static __global__ void __launch_bounds__(kThreads, 1) apsp_batch_levels_kernel(const BatchArgs b, unsigned long long* lists,
+                                                                        size_t list_words) {
+  __shared__ ApspSmem sm;
+  extern __shared__ __align__(16) unsigned s_dyn[];
+  const int team = (int)blockIdx.x / b.team_ctas, cta = (int)blockIdx.x % b.team_ctas;
+  if (team >= b.n_teams) return;
+  if (b.stop && ld_volatile_i32(b.stop) != 0) return;   // written before the launch: the same in every CTA
+  if (threadIdx.x < 8) sm.seen[threadIdx.x >> 1][threadIdx.x & 1] = 0ULL;
+  __syncthreads();
+  unsigned long long* const words = lists + (size_t)team * list_words;
+  LevelsList ws;
+  ws.list = words;
+  ws.hash = words + kLevelsList;
+  ws.hlev = reinterpret_cast<unsigned char*>(words + 3 * (size_t)kLevelsList);
+  ws.counters = reinterpret_cast<unsigned*>(words + kLevelsListWords);
+  ApspArgs a;
+  a.adj2 = nullptr;
+  a.ctrl = b.team_ctrl + team;
+  a.timeout_ns = b.timeout_ns;
+  uint4* const m0 = b.scratch + b.team_off[team];
+  uint4* const m1 = m0 + b.team_cells[team];
+  unsigned long long bar_target = 0;
+  unsigned gl = 0;
+  const int k0 = b.team_start[team], k1 = b.team_start[team + 1];
+  for (int k = k0; k < k1; ++k) {
+    const int gi = b.team_list[k];
+    const BatchGraph gr = b.graphs[gi];
+    a.adj = gr.adj;
+    a.N = gr.N;
+    a.d = gr.d;
+    a.vec4 = gr.vec4;
+    EvalOut o;
+    const int r = eval_levels(a, ws, (unsigned)(k - k0), m0, m1, cta, b.team_ctas, sm, s_dyn, bar_target, gl, o);
+    if (r == kLevelsFailed) {
+      if (b.sticky && threadIdx.x == 0) atomicCAS(b.sticky, 0, max(1, ld_volatile_i32(&a.ctrl->error)));
+      return;
+    }
+    if (r == kLevelsDone && cta == 0 && threadIdx.x == 0) {
+      BatchOut* w = b.out + gi;
+      w->sum = o.sum;
+      w->levels = o.levels;
+      w->dense_levels = o.dense_levels;
+      w->diam = o.diam;
+      w->disconnected = o.disconnected;
+      w->windows = o.windows;
+      w->error = 0;
+      w->done = 1;
+    }
+  }
 }
 
 }  // namespace ggb

@@ -86,32 +86,25 @@ struct SliceTotals {
   int levels = 0, diam = 1, disconnected = 0, windows = 0;
 };
 
-__device__ __forceinline__ void slice_finish(const SliceArgs& a, const SliceTotals& r) {
+// Adds a CTA's totals to the record; the last of n_ctas hands the whole to
+// write(sum, levels, windows, diam, disconnected, error, info) and clears it.
+template <typename Write>
+__device__ __forceinline__ void slice_finish(ApspCtrl* c, int groups, unsigned n_ctas, const SliceTotals& r,
+                                             Write write) {
   if (threadIdx.x != 0) return;
-  ApspCtrl* c = a.ctrl;
-  const unsigned long long sum = r.s1_lo * (unsigned)a.groups + r.s1_hi * 2u * (unsigned)a.groups + r.s2;
+  const unsigned long long sum = r.s1_lo * (unsigned)groups + r.s1_hi * 2u * (unsigned)groups + r.s2;
   atomicAdd(reinterpret_cast<unsigned long long*>(&c->sum), sum);
   atomicAdd(reinterpret_cast<unsigned long long*>(&c->levels), (unsigned long long)r.levels);
   atomicMax(&c->diam, r.diam);
   if (r.disconnected) atomicOr(&c->disconnected, 1);
   atomicAdd(&c->windows, r.windows);
   __threadfence();
-  if (atomicAdd(&c->bar, 1ULL) != (unsigned long long)gridDim.x - 1) return;
+  if (atomicAdd(&c->bar, 1ULL) != (unsigned long long)n_ctas - 1) return;
   __threadfence();
   const int err = __ldcg(&c->error), info = __ldcg(&c->error_info), dm = __ldcg(&c->diam);
   const int dc = __ldcg(&c->disconnected), nw = __ldcg(&c->windows);
   const long long sm = __ldcg(&c->sum), lv = __ldcg(&c->levels);
-  ApspCtrl* o = a.out;
-  o->error = err;
-  o->error_info = info;
-  o->diam = dm;
-  o->disconnected = dc;
-  o->sum = sm;
-  o->levels = lv;
-  o->dense_levels = lv - nw;
-  o->windows = nw;
-  o->trace_len = 0;
-  o->done = 1;
+  write(sm, lv, nw, dm, dc, err, info);
   c->error = 0;
   c->error_info = 0;
   c->diam = 0;
@@ -122,6 +115,24 @@ __device__ __forceinline__ void slice_finish(const SliceArgs& a, const SliceTota
   c->asym = 0;
   c->cnt[0][0] = 0ULL;
   c->bar = 0ULL;
+}
+
+// The record of a single evaluation, in pinned host memory.
+__device__ __forceinline__ void slice_finish(const SliceArgs& a, const SliceTotals& r) {
+  slice_finish(a.ctrl, a.groups, gridDim.x, r, [&](long long sum, long long levels, int windows, int diam,
+                                                   int disconnected, int error, int info) {
+    ApspCtrl* o = a.out;
+    o->error = error;
+    o->error_info = info;
+    o->diam = diam;
+    o->disconnected = disconnected;
+    o->sum = sum;
+    o->levels = levels;
+    o->dense_levels = levels - windows;
+    o->windows = windows;
+    o->trace_len = 0;
+    o->done = 1;
+  });
 }
 
 // ---- small graphs: every vertex at every level ----------------------------------
@@ -140,8 +151,9 @@ __device__ __forceinline__ void slice_finish(const SliceArgs& a, const SliceTota
 // Shared memory: two row buffers and the adjacency.
 inline size_t slice_smem_bytes(int np, int words, int pairs) { return (size_t)np * (words * 8 + pairs * 4); }
 
+// Windows t0, t0 + step, ... below t1 of one graph on this CTA.
 template <int WORDS>
-__global__ void __launch_bounds__(1024, 1) slice_kernel(const SliceArgs a) {
+__device__ __forceinline__ SliceTotals slice_windows(const SliceArgs& a, int t0, int t1, int step) {
   using Row = SliceRow<WORDS>;
   using T = typename Row::T;
   extern __shared__ __align__(16) unsigned char s_raw[];
@@ -170,7 +182,7 @@ __global__ void __launch_bounds__(1024, 1) slice_kernel(const SliceArgs a) {
 
   SliceTotals r;
   unsigned g = 0;                      // levels run so far: the rotation of s_cnt
-  for (int t = blockIdx.x; t < a.nw1 + a.nw2 && !r.disconnected; t += gridDim.x) {
+  for (int t = t0; t < t1 && !r.disconnected; t += step) {
     const int phase = t < a.nw1 ? 1 : 2;
     const int first = (phase == 1 ? t : t - a.nw1) * a.width;
     const int l = min(a.width, (phase == 1 ? a.n_src1 : a.ac) - first);
@@ -234,7 +246,57 @@ __global__ void __launch_bounds__(1024, 1) slice_kernel(const SliceArgs a) {
     if (act == 2) { r.disconnected = 1; r.diam = N + 1; }
     else r.diam = max(r.diam, kk + 1);
   }
-  slice_finish(a, r);
+  return r;
+}
+
+template <int WORDS>
+__global__ void __launch_bounds__(1024, 1) slice_kernel(const SliceArgs a) {
+  slice_finish(a, slice_windows<WORDS>(a, (int)blockIdx.x, a.nw1 + a.nw2, (int)gridDim.x));
+}
+
+// ---- many small graphs, one launch ---------------------------------------------------
+// CTA i takes the windows items[i] of one graph of a batch (see BatchGraph);
+// each graph has a record of its own, and the last of its CTAs writes its
+// BatchOut.  Nothing to clear before the launch.
+template <int WORDS>
+__global__ void __launch_bounds__(1024, 1) slice_batch_kernel(const BatchGraph* __restrict__ graphs,
+                                                              const SliceItem* __restrict__ items,
+                                                              ApspCtrl* __restrict__ records, BatchOut* __restrict__ out,
+                                                              const int* stop, int* sticky) {
+  if (stop && ld_volatile_i32(stop) != 0) return;   // written before the launch: the same in every CTA
+  const SliceItem it = items[blockIdx.x];
+  const BatchGraph gr = graphs[it.graph];
+  SliceArgs a;
+  a.adj = gr.adj;
+  a.adj16 = nullptr;
+  a.deg = nullptr;
+  a.ctrl = records + it.graph;
+  a.out = nullptr;
+  a.N = gr.N;
+  a.d = gr.d;
+  a.pairs = (gr.d + 1) / 2;
+  a.np = (gr.N + 31) / 32 * 32;
+  a.n_src1 = gr.n_src;
+  a.split = gr.N;
+  a.ac = 0;
+  a.groups = gr.groups;
+  a.width = 32 * WORDS;
+  a.nw1 = (gr.n_src + a.width - 1) / a.width;
+  a.nw2 = 0;
+  const SliceTotals r = slice_windows<WORDS>(a, it.first, it.end, 1);
+  slice_finish(a.ctrl, gr.groups, (unsigned)it.ctas, r, [&](long long sum, long long levels, int windows, int diam,
+                                                            int disconnected, int error, int) {
+    BatchOut* o = out + it.graph;
+    o->sum = sum;
+    o->levels = levels;
+    o->dense_levels = levels - windows;
+    o->diam = diam;
+    o->disconnected = disconnected;
+    o->windows = windows;
+    o->error = error;
+    o->done = error ? 0 : 1;
+    if (error && sticky) atomicCAS(sticky, 0, error);
+  });
 }
 
 // ---- lattice graphs: rings of new bits -----------------------------------------
@@ -272,7 +334,7 @@ __device__ __forceinline__ int strip_source(int i, int H, int n) {
   return (rem / hs) * H + s * kStripRows + rem % hs;
 }
 
-__global__ void __launch_bounds__(1024, 1) slice_push_kernel(const SliceArgs a) {
+static __global__ void __launch_bounds__(1024, 1) slice_push_kernel(const SliceArgs a) {
   extern __shared__ __align__(16) unsigned char s_raw[];
   __shared__ unsigned s_cnt[3];        // new bits of a level, in rotation
   __shared__ unsigned s_n[3];          // vertices that received bits, in rotation
@@ -464,7 +526,7 @@ __global__ void lattice_prep_kernel(const ID* __restrict__ adj, const int* __res
 // H + (r - 1): the middle of the second run of differences is H.  A numbering
 // without that structure gives H = n_src (the sources in id order).  Clears
 // diff[] for the next launch.
-__global__ void __launch_bounds__(1024) lattice_height_kernel(const int* __restrict__ inv, unsigned* __restrict__ diff,
+static __global__ void __launch_bounds__(1024) lattice_height_kernel(const int* __restrict__ inv, unsigned* __restrict__ diff,
                                                               int N, int n_src, int* __restrict__ height,
                                                               ApspCtrl* ctrl) {
   __shared__ int s_at[3];              // first gap, first difference past it, first gap past that

@@ -42,6 +42,26 @@ struct ggb_batch {
   long long* d_tsoff = nullptr;      // [max_teams]
   unsigned* d_stamps = nullptr;
   size_t cap_stamps = 0;             // unsigned
+  // The automatic plan splits the graphs over three kernels: small ones on
+  // shared-memory windows (apsp_slice.cuh), mid-size ones level by level on
+  // teams (apsp_levels.cuh), the rest on teams of windows as a fixed plan has
+  // them all.
+  bool split = false;
+  struct SliceLaunch { int words, threads, first, items; size_t smem; };
+  std::vector<SliceLaunch> slices;          // by shared memory, so that small graphs share an SM
+  std::vector<ggb::SliceItem> slice_items;
+  std::vector<int> slice_words;             // per graph: row words of its slices, 0: not a slice graph
+  ggb::SliceItem* d_items = nullptr;  size_t cap_items = 0;
+  ggb::ApspCtrl* d_records = nullptr;       // [n], all zero between launches
+  int lT = 0, l_teams = 0;                  // level-by-level teams (l_teams == 0: none)
+  size_t l_smem = 0;
+  std::vector<int> l_start, l_list;
+  std::vector<long long> l_off, l_cells;
+  int* d_lint = nullptr;      size_t cap_lint = 0;       // l_start, l_list
+  long long* d_lll = nullptr; size_t cap_lll = 0;        // l_off, l_cells
+  ggb::ApspCtrl* d_lctrl = nullptr;         // [2 * max_teams]: the teams, then the window launch behind them
+  ggb::ApspCtrl* h_lctrl = nullptr;
+  unsigned long long* d_lists = nullptr; size_t cap_lists = 0;
   int occ[6] = {0, 0, 0, 0, 0, 0};   // co-resident batch CTAs per SM, per log2(R)
   int max_teams = 0;                 // largest CTA count of any plan
   long long timeout_ns = 2000000000LL;
