@@ -19,10 +19,10 @@
 // operands staged in shared memory by bulk copies, bias, ReLU and the output
 // head applied between tcgen05.ld and the next product, no round trip through
 // global memory.  It replaced an mma.sync kernel of the same fusion (ldmatrix
-// fragments, 32 rows a CTA): 8.2 us against 10.3 us for 4096 rows.  The
-// training products (at most 256 rows, with the pre-activations the backward
-// needs) are one warp per 16 x 8 output tile issuing mma.sync.m16n8k16 (BF16
-// in, FP32 accumulate) on operands read straight from L2.
+// fragments, 32 rows a CTA): 8.2 us against 10.3 us for 4096 rows.  A
+// training step (at most 256 rows) is two launches of mma.sync.m16n8k16 (BF16
+// in, FP32 accumulate): train_rows_kernel does all that is local to 16 rows,
+// train_weights_kernel the sums over the rows and Adam.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -51,8 +51,6 @@ namespace mlp {
 
 using bf16 = __nv_bfloat16;
 
-__device__ __forceinline__ uint32_t ld_pair(const bf16* p) { return *reinterpret_cast<const uint32_t*>(p); }
-
 // D = A (16x16, row) * B (16x8, col) + D, BF16 inputs, FP32 accumulators.
 __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                           uint32_t b0, uint32_t b1) {
@@ -61,65 +59,6 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
       "{%0,%1,%2,%3};\n"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-enum Epi : int {
-  kEpiBiasReluBf16 = 0,   // out_b[m][n] = bf16(relu(c + bias[n]))
-  kEpiBiasReluF32 = 1,    // out_f[m][n] = relu(c + bias[n]); out_z[m][n] = c + bias[n] (if out_z)
-  kEpiF32 = 2,            // out_f[m][n] = c
-  kEpiMask = 3,           // v = c * (mask[m][n] > 0): out_b = bf16(v), out_f = v
-};
-
-struct EpiArgs {
-  const float* bias;
-  const bf16* mask;       // [M][N]
-  bf16* out_b;
-  float* out_f;
-  float* out_z;
-};
-
-// C[M][N] = A[M][K] * Bt[N][K]^T with the epilogue EPI; M % 16 == 0,
-// N % 8 == 0, K % 16 == 0, lda/ldb even.  One warp per 16 x 8 tile.
-template <int EPI>
-__global__ void __launch_bounds__(128) gemm_tn_kernel(int M, int N, int K, const bf16* __restrict__ A, int lda,
-                                                      const bf16* __restrict__ Bt, int ldb, EpiArgs e) {
-  const int lane = threadIdx.x & 31;
-  const long long tile = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
-  const int tiles_n = N / 8;
-  if (tile >= (long long)(M / 16) * tiles_n) return;
-  const int m0 = (int)(tile / tiles_n) * 16, n0 = (int)(tile % tiles_n) * 8;
-  const int g = lane >> 2, t = lane & 3;
-  float c[4] = {0.f, 0.f, 0.f, 0.f};
-  const bf16* a_r0 = A + (long long)(m0 + g) * lda + 2 * t;
-  const bf16* a_r1 = a_r0 + 8LL * lda;
-  const bf16* b_n = Bt + (long long)(n0 + g) * ldb + 2 * t;
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    const uint32_t a0 = ld_pair(a_r0 + k0), a1 = ld_pair(a_r1 + k0);
-    const uint32_t a2 = ld_pair(a_r0 + k0 + 8), a3 = ld_pair(a_r1 + k0 + 8);
-    const uint32_t b0 = ld_pair(b_n + k0), b1 = ld_pair(b_n + k0 + 8);
-    mma_16816(c, a0, a1, a2, a3, b0, b1);
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + g + (i >= 2 ? 8 : 0);
-    const int n = n0 + 2 * t + (i & 1);
-    const long long o = (long long)m * N + n;
-    float v = c[i];
-    if (EPI == kEpiBiasReluBf16) {
-      v += e.bias[n];
-      e.out_b[o] = __float2bfloat16_rn(v > 0.f ? v : 0.f);
-    } else if (EPI == kEpiBiasReluF32) {
-      v += e.bias[n];
-      if (e.out_z) e.out_z[o] = v;
-      e.out_f[o] = v > 0.f ? v : 0.f;
-    } else if (EPI == kEpiF32) {
-      e.out_f[o] = v;
-    } else {
-      v = __bfloat162float(e.mask[o]) > 0.f ? v : 0.f;
-      e.out_b[o] = __float2bfloat16_rn(v);
-      e.out_f[o] = v;
-    }
-  }
 }
 
 // Bulk copies global -> shared (cp.async.bulk, completion on an mbarrier).
@@ -383,137 +322,389 @@ __global__ void __launch_bounds__(tc::kThreads, 1) forward_tc_kernel(const bf16*
   }
 }
 
-// y[r] = H2[r][:] . w3 + b3 (one warp per row, fixed summation order).
-__global__ void head_kernel(const float* __restrict__ H2, const float* __restrict__ w3, const float* __restrict__ b3,
-                            float* __restrict__ y, int rows) {
-  const int lane = threadIdx.x & 31;
-  const long long r = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (r >= rows) return;
-  float s = 0.f;
-  for (int n = lane; n < kHidden; n += 32) s = fmaf(H2[r * kHidden + n], w3[n], s);
+// ---- the training step -----------------------------------------------------------------
+// Four 8 x 8 BF16 matrices, one 16-byte row address a lane (lane 8i + r: row r
+// of matrix i); TRANS: each transposed.
+template <bool TRANS>
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], unsigned saddr) {
+  if constexpr (TRANS)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(saddr)
+                 : "memory");
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(saddr)
+                 : "memory");
+}
+
+// acc[nt] += A (16 rows, columns of A) * B^T for this warp's four column tiles
+// n0 + 8 nt, over K columns in steps of 16 in ascending order.  A and W lie in
+// shared memory in the operand layout (umma_k_off), whose core matrices are
+// ldmatrix's 8 x 8 matrices, so every access is free of bank conflicts.
+// TRANS false: B[n][k] = W[n][k], W of KW columns.  TRANS true: B[n][k] = W[k][n].
+template <bool TRANS>
+__device__ __forceinline__ void warp_product(float (&acc)[4][4], const bf16* A, int KA, const bf16* W, int KW, int n0,
+                                             int K) {
+  const int lane = threadIdx.x & 31, i = lane >> 3, r = lane & 7;
+  for (int k0 = 0; k0 < K; k0 += 16) {
+    // A fragment: (rows 0-7, k 0-7), (rows 8-15, k 0-7), (rows 0-7, k 8-15), (rows 8-15, k 8-15)
+    uint32_t a[4];
+    ldmatrix4<false>(a, smem_u32(A + umma_k_off(8 * (i & 1) + r, k0 + 8 * (i >> 1), KA)));
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) y[r] = s + b3[0];
-}
-
-// Backward through the output layer for B rows: dy, dZ2 (BF16, both
-// layouts), the gradients of w3, b3 and b2, and the loss.  One block of 256
-// threads: thread n owns hidden unit n.
-__global__ void __launch_bounds__(kHidden) out_backward_kernel(const float* __restrict__ y,
-                                                               const float* __restrict__ t,
-                                                               const float* __restrict__ Z2,
-                                                               const float* __restrict__ H2,
-                                                               const float* __restrict__ w3, int B,
-                                                               bf16* __restrict__ dZ2, bf16* __restrict__ dZ2t,
-                                                               float* __restrict__ grad, float* __restrict__ loss) {
-  __shared__ float s_dy[kMaxTrainRows];
-  const int n = threadIdx.x;
-  for (int r = n; r < B; r += kHidden) s_dy[r] = 2.f * (y[r] - t[r]) / (float)B;
-  __syncthreads();
-  const float wn = w3[n];
-  float gw3 = 0.f, gb2 = 0.f;
-  for (int r = 0; r < B; ++r) {
-    const float dy = s_dy[r];
-    gw3 = fmaf(dy, H2[(long long)r * kHidden + n], gw3);
-    const float dz = Z2[(long long)r * kHidden + n] > 0.f ? dy * wn : 0.f;
-    const bf16 db = __float2bfloat16_rn(dz);
-    dZ2[(long long)r * kHidden + n] = db;
-    dZ2t[(long long)n * B + r] = db;
-    gb2 += dz;
-  }
-  grad[kOffW3 + n] = gw3;
-  grad[kOffB2 + n] = gb2;
-  if (n == 0) {
-    float gb3 = 0.f, l = 0.f;
-    for (int r = 0; r < B; ++r) {
-      gb3 += s_dy[r];
-      const float d = y[r] - t[r];
-      l = fmaf(d, d, l);
+    for (int p = 0; p < 2; ++p) {      // two column tiles a load
+      const int n = n0 + 16 * p;
+      uint32_t b[4];
+      if constexpr (TRANS)
+        ldmatrix4<true>(b, smem_u32(W + umma_k_off(k0 + 8 * (i & 1) + r, n + 8 * (i >> 1), KW)));
+      else
+        ldmatrix4<false>(b, smem_u32(W + umma_k_off(n + 8 * (i >> 1) + r, k0 + 8 * (i & 1), KW)));
+      mma_16816(acc[2 * p], a[0], a[1], a[2], a[3], b[0], b[1]);
+      mma_16816(acc[2 * p + 1], a[0], a[1], a[2], a[3], b[2], b[3]);
     }
-    grad[kOffB3] = gb3;
-    if (loss) *loss = l / (float)B;
   }
 }
 
-// out[c][r] = in[r][c] for a rows x cols BF16 matrix.
-__global__ void transpose_bf16_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, int rows, int cols) {
-  const long long n = (long long)rows * cols;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const int r = (int)(i / cols), c = (int)(i % cols);
-    out[(long long)c * rows + r] = in[i];
+namespace tr {
+constexpr int kRows = 16;                                  // rows a CTA of the row pass
+constexpr int kThreads = 256;
+constexpr uint32_t kSW1 = kHidden * kHidden * 2;          // behind W2
+constexpr uint32_t kSX = kSW1 + kHidden * kFeatures * 2;
+constexpr uint32_t kSH1 = kSX + kRows * kFeatures * 2;
+constexpr uint32_t kSD2 = kSH1 + kRows * kHidden * 2;
+constexpr int kPitch = kHidden + 4;                        // FP32 rows of H2, off the banks of the row before
+constexpr uint32_t kSH2 = kSD2 + kRows * kHidden * 2;
+constexpr uint32_t kSDy = kSH2 + kRows * kPitch * 4;
+constexpr size_t kSmem = kSDy + kRows * 4;
+}  // namespace tr
+
+// Everything of a training step that is local to a row, 16 rows a CTA: both
+// layers, the head, the output error, and the gradients entering both hidden
+// layers.  W1 and W2 are staged once by bulk copies (W2 serves the second layer
+// and, transposed by ldmatrix, its backward).  Writes H1, H2, dZ2, dZ1 and the
+// errors for train_weights_kernel.  With count, CTA 0 advances the Adam step.
+//
+// Bound: the chain staging -> layer 1 -> layer 2 -> head -> dZ2 -> dZ1 on a few
+// CTAs.  The two kernels replaced thirteen launches (products, head, the output
+// layer's backward on one block, transposes, sums, Adam and its counter): eight
+// steps on 64 rows, with the copies to and from the host around them, took
+// 765 us and take 206.
+__global__ void __launch_bounds__(tr::kThreads, 1) train_rows_kernel(const bf16* __restrict__ X,
+                                                                   const int* __restrict__ idx,
+                                                                   const float* __restrict__ t, int B,
+                                                                   const bf16* __restrict__ W1u,
+                                                                   const bf16* __restrict__ W2u,
+                                                                   const float* __restrict__ params,
+                                                                   bf16* __restrict__ H1, float* __restrict__ H2,
+                                                                   bf16* __restrict__ dZ2, bf16* __restrict__ dZ1,
+                                                                   float* __restrict__ dZ1f, float* __restrict__ err,
+                                                                   int* __restrict__ step, int count) {
+  using namespace tr;
+  extern __shared__ __align__(1024) unsigned char s_tr[];
+  __shared__ alignas(8) unsigned long long s_bars[2];      // W1 staged, W2 staged
+  bf16* const W2s = reinterpret_cast<bf16*>(s_tr);
+  bf16* const W1s = reinterpret_cast<bf16*>(s_tr + kSW1);
+  bf16* const Xs = reinterpret_cast<bf16*>(s_tr + kSX);
+  bf16* const H1s = reinterpret_cast<bf16*>(s_tr + kSH1);
+  bf16* const D2s = reinterpret_cast<bf16*>(s_tr + kSD2);
+  float* const H2s = reinterpret_cast<float*>(s_tr + kSH2);
+  float* const dys = reinterpret_cast<float*>(s_tr + kSDy);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g = lane >> 2, q = lane & 3;                   // accumulator rows g, g + 8, columns 2q, 2q + 1
+  const int r0 = blockIdx.x * kRows, n0 = 32 * warp;
+  const unsigned bar1 = smem_u32(&s_bars[0]), bar2 = smem_u32(&s_bars[1]);
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar1) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar2) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    constexpr uint32_t w1 = kHidden * kFeatures * 2, w2 = kHidden * kHidden * 2;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar1), "r"(w1) : "memory");
+    bulk_copy(W1s, W1u, w1, bar1);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar2), "r"(w2) : "memory");
+    for (uint32_t c = 0; c < w2; c += 16384u)
+      bulk_copy(s_tr + c, reinterpret_cast<const unsigned char*>(W2u) + c, 16384u, bar2);
+    if (count && blockIdx.x == 0) *step += 1;
   }
+  if (tid < kRows * (kFeatures / 8)) {
+    const int r = tid / (kFeatures / 8), c = (tid % (kFeatures / 8)) * 8;
+    const int src = idx ? idx[r0 + r] : r0 + r;
+    *reinterpret_cast<uint4*>(Xs + umma_k_off(r, c, kFeatures)) =
+        *reinterpret_cast<const uint4*>(X + (long long)src * kFeatures + c);
+  }
+  float b1v[4][2], b2v[4][2];
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      b1v[nt][e] = params[kOffB1 + n0 + 8 * nt + 2 * q + e];
+      b2v[nt][e] = params[kOffB2 + n0 + 8 * nt + 2 * q + e];
+    }
+  const float w3n = params[kOffW3 + tid], b3 = params[kOffB3];
+  float w3l[kHidden / 32];
+#pragma unroll
+  for (int i = 0; i < kHidden / 32; ++i) w3l[i] = params[kOffW3 + lane + 32 * i];
+  __syncthreads();
+  // layer 1
+  bool ok = mbar_wait_bounded(bar1, 0u);
+  float acc[4][4];
+  auto clear = [&]() {
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[nt][i] = 0.f;
+  };
+  clear();
+  warp_product<false>(acc, Xs, kFeatures, W1s, kFeatures, n0, kFeatures);
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = g + 8 * h, n = n0 + 8 * nt + 2 * q;
+      const float v0 = acc[nt][2 * h] + b1v[nt][0], v1 = acc[nt][2 * h + 1] + b1v[nt][1];
+      __nv_bfloat162 o;
+      o.x = __float2bfloat16_rn(v0 > 0.f ? v0 : 0.f);
+      o.y = __float2bfloat16_rn(v1 > 0.f ? v1 : 0.f);
+      *reinterpret_cast<__nv_bfloat162*>(H1s + umma_k_off(r, n, kHidden)) = o;
+      *reinterpret_cast<__nv_bfloat162*>(H1 + (size_t)(r0 + r) * kHidden + n) = o;
+    }
+  __syncthreads();
+  // layer 2
+  ok = mbar_wait_bounded(bar2, 0u) && ok;
+  clear();
+  warp_product<false>(acc, H1s, kHidden, W2s, kHidden, n0, kHidden);
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = g + 8 * h, n = n0 + 8 * nt + 2 * q;
+      const float v0 = acc[nt][2 * h] + b2v[nt][0], v1 = acc[nt][2 * h + 1] + b2v[nt][1];
+      const float2 o = make_float2(v0 > 0.f ? v0 : 0.f, v1 > 0.f ? v1 : 0.f);
+      *reinterpret_cast<float2*>(H2s + r * kPitch + n) = o;
+      *reinterpret_cast<float2*>(H2 + (size_t)(r0 + r) * kHidden + n) = o;
+    }
+  __syncthreads();
+  // head: y = H2 . w3 + b3, one warp per row; then the output error
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = warp + 8 * h;
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < kHidden / 32; ++i) s = fmaf(H2s[r * kPitch + lane + 32 * i], w3l[i], s);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+      const float y = s + b3;
+      const float d = y - t[r0 + r];
+      const float dy = 2.f * d / (float)B;
+      dys[r] = dy;
+      err[r0 + r] = ok ? dy : __int_as_float(0x7fc00000);
+      err[kMaxTrainRows + r0 + r] = d;
+    }
+  }
+  __syncthreads();
+  // dZ2: thread n owns hidden unit n
+#pragma unroll 4
+  for (int r = 0; r < kRows; ++r) {
+    const bf16 db = __float2bfloat16_rn(H2s[r * kPitch + tid] > 0.f ? dys[r] * w3n : 0.f);
+    D2s[umma_k_off(r, tid, kHidden)] = db;
+    dZ2[(size_t)(r0 + r) * kHidden + tid] = db;
+  }
+  __syncthreads();
+  // dZ1 = (dZ2 W2) where H1 > 0
+  clear();
+  warp_product<true>(acc, D2s, kHidden, W2s, kHidden, n0, kHidden);
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = g + 8 * h, n = n0 + 8 * nt + 2 * q;
+      const __nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162*>(H1s + umma_k_off(r, n, kHidden));
+      const float v0 = __bfloat162float(m.x) > 0.f ? acc[nt][2 * h] : 0.f;
+      const float v1 = __bfloat162float(m.y) > 0.f ? acc[nt][2 * h + 1] : 0.f;
+      __nv_bfloat162 o;
+      o.x = __float2bfloat16_rn(v0);
+      o.y = __float2bfloat16_rn(v1);
+      const size_t at = (size_t)(r0 + r) * kHidden + n;
+      *reinterpret_cast<__nv_bfloat162*>(dZ1 + at) = o;
+      *reinterpret_cast<float2*>(dZ1f + at) = make_float2(v0, v1);
+    }
 }
 
-// grad[off + c] = sum_r in[r][c] (fixed order).
-__global__ void col_sum_kernel(const float* __restrict__ in, int rows, int cols, float* __restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float s = 0.f;
-  for (int r = 0; r < rows; ++r) s += in[(long long)r * cols + c];
-  out[c] = s;
-}
-
-// The BF16 copies of parameter i (value v) that the products read: W1 and
-// W2 row-major, W2 transposed, and W1 / W2 in the tcgen05 operand layout.
-__device__ __forceinline__ void store_bf16_copies(int i, float v, bf16* __restrict__ w1b, bf16* __restrict__ w2b,
-                                                  bf16* __restrict__ w2tb, bf16* __restrict__ w1u,
-                                                  bf16* __restrict__ w2u) {
-  const bf16 b = __float2bfloat16_rn(v);
+// The BF16 copies of parameter i (value v) that the products read: W1 and W2
+// in the operand layout.
+__device__ __forceinline__ void store_bf16_copies(int i, float v, bf16* __restrict__ w1u, bf16* __restrict__ w2u) {
   if (i < kOffB1) {
-    w1b[i] = b;
-    w1u[umma_k_off(i / kFeatures, i % kFeatures, kFeatures)] = b;
+    w1u[umma_k_off(i / kFeatures, i % kFeatures, kFeatures)] = __float2bfloat16_rn(v);
   } else if (i >= kOffW2 && i < kOffB2) {
-    const int q = i - kOffW2, n = q / kHidden, k = q % kHidden;
-    w2b[q] = b;
-    w2tb[k * kHidden + n] = b;
-    w2u[umma_k_off(n, k, kHidden)] = b;
+    const int q = i - kOffW2;
+    w2u[umma_k_off(q / kHidden, q % kHidden, kHidden)] = __float2bfloat16_rn(v);
   }
 }
 
-// Adam on the FP32 master parameters, then the BF16 copies the products
-// read (W1, W2 and W2 transposed).  The step counter lives on the device so
-// that a replayed graph keeps counting; adam_step_kernel advances it after
-// every block of this kernel has used it.
-__global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m1,
-                            float* __restrict__ m2, const int* __restrict__ step, AdamHyper h, bf16* __restrict__ w1b,
-                            bf16* __restrict__ w2b, bf16* __restrict__ w2tb, bf16* __restrict__ w1u,
-                            bf16* __restrict__ w2u) {
-  const int t = *step + 1;
-  const float c1 = 1.f / (1.f - powf(h.beta1, (float)t));
-  const float c2 = 1.f / (1.f - powf(h.beta2, (float)t));
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x) {
-    const float gi = g[i];
-    const float a = h.beta1 * m1[i] + (1.f - h.beta1) * gi;
-    const float b = h.beta2 * m2[i] + (1.f - h.beta2) * gi * gi;
-    m1[i] = a;
-    m2[i] = b;
-    const float pi = p[i] - h.lr * (a * c1) / (sqrtf(b * c2) + h.eps);
-    p[i] = pi;
-    store_bf16_copies(i, pi, w1b, w2b, w2tb, w1u, w2u);
+// What becomes of a gradient: written out, or one Adam step on the FP32 master
+// parameter (the step count was advanced by the row pass) and its BF16 copies.
+struct GradSink {
+  float* g;                  // null: Adam
+  float *p, *m1, *m2;
+  const int* step;
+  AdamHyper h;
+  bf16 *w1u, *w2u;
+};
+
+struct AdamScale {
+  float c1, c2;
+  __device__ __forceinline__ explicit AdamScale(const GradSink& s) {
+    const int t = s.g ? 1 : *s.step;
+    c1 = 1.f / (1.f - powf(s.h.beta1, (float)t));
+    c2 = 1.f / (1.f - powf(s.h.beta2, (float)t));
   }
+};
+
+__device__ __forceinline__ void sink_gradient(const GradSink& s, const AdamScale& c, int i, float gi, float m1i,
+                                              float m2i, float p0) {
+  if (s.g) {
+    s.g[i] = gi;
+    return;
+  }
+  const float a = s.h.beta1 * m1i + (1.f - s.h.beta1) * gi;
+  const float b = s.h.beta2 * m2i + (1.f - s.h.beta2) * gi * gi;
+  s.m1[i] = a;
+  s.m2[i] = b;
+  const float pi = p0 - s.h.lr * (a * c.c1) / (sqrtf(b * c.c2) + s.h.eps);
+  s.p[i] = pi;
+  store_bf16_copies(i, pi, s.w1u, s.w2u);
 }
 
-__global__ void adam_step_kernel(int* step) { *step += 1; }
+// The sums over the rows, and what becomes of them.  Blocks 0 .. 127: 16 x 32
+// tiles of gW2[n][k] = sum_r dZ2[r][n] H1[r][k], a 16 x 8 tile a warp; blocks
+// 128 .. 143: 16 x 32 rows of gW1[k][j] = sum_r dZ1[r][k] X[r][j]; block 144:
+// the FP32 sums of w3, b2, b3 and the loss; block 145: b1.  The products run
+// over r in steps of 16, the sums one row after the other.  The operands are
+// staged row by row and transposed by ldmatrix, so no transposed copy exists.
+constexpr int kWeightBlocks = 146;
+__global__ void __launch_bounds__(128) train_weights_kernel(const bf16* __restrict__ X, const int* __restrict__ idx,
+                                                            int B, const bf16* __restrict__ H1,
+                                                            const float* __restrict__ H2,
+                                                            const bf16* __restrict__ dZ2,
+                                                            const bf16* __restrict__ dZ1,
+                                                            const float* __restrict__ dZ1f,
+                                                            const float* __restrict__ err, GradSink s,
+                                                            float* __restrict__ loss) {
+  // rows of 16 + 8 and 32 + 8 columns: ldmatrix's eight rows fall on different banks
+  constexpr int kPA = 24, kPB = 40;
+  __shared__ __align__(16) bf16 As[kMaxTrainRows * kPA];
+  __shared__ __align__(16) bf16 Bs[kMaxTrainRows * kPB];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int blk = blockIdx.x;
+  if (blk < 144) {
+    const bool w2 = blk < 128;
+    const int m0 = w2 ? (blk >> 3) * 16 : (blk - 128) * 16;   // rows of the gradient
+    const int c0 = w2 ? (blk & 7) * 32 : 0;                   // its first column here
+    const int ld = w2 ? kHidden : kFeatures, off = w2 ? kOffW2 : kOffW1;
+    const bf16* const A = w2 ? dZ2 : dZ1;
+    for (int i = tid; i < B * 2; i += 128)
+      *reinterpret_cast<uint4*>(As + (i >> 1) * kPA + 8 * (i & 1)) =
+          *reinterpret_cast<const uint4*>(A + (size_t)(i >> 1) * kHidden + m0 + 8 * (i & 1));
+    for (int i = tid; i < B * 4; i += 128) {
+      const int r = i >> 2;
+      const bf16* row = w2 ? H1 + (size_t)r * kHidden + c0 : X + (long long)(idx ? idx[r] : r) * kFeatures;
+      *reinterpret_cast<uint4*>(Bs + r * kPB + 8 * (i & 3)) = *reinterpret_cast<const uint4*>(row + 8 * (i & 3));
+    }
+    // the parameters this lane will update, while the rows arrive
+    const int gr = lane >> 2, q = lane & 3, n0 = 8 * warp;
+    int at[4];
+    float m1v[4], m2v[4], pv[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      at[i] = off + (m0 + gr + (i >= 2 ? 8 : 0)) * ld + c0 + n0 + 2 * q + (i & 1);
+      if (!s.g) {
+        m1v[i] = s.m1[at[i]];
+        m2v[i] = s.m2[at[i]];
+        pv[i] = s.p[at[i]];
+      } else {
+        m1v[i] = m2v[i] = pv[i] = 0.f;
+      }
+    }
+    const AdamScale c(s);
+    __syncthreads();
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    const int i = lane >> 3, r = lane & 7;
+    for (int k0 = 0; k0 < B; k0 += 16) {
+      // A[m][k] = As[k][m]: (m 0-7, k 0-7), (m 8-15, k 0-7), (m 0-7, k 8-15), (m 8-15, k 8-15)
+      uint32_t a[4], b[4];
+      ldmatrix4<true>(a, smem_u32(As + (k0 + 8 * (i >> 1) + r) * kPA + 8 * (i & 1)));
+      // B[k][n] = Bs[k][n]: (k 0-7), (k 8-15); the other two addresses repeat them
+      ldmatrix4<true>(b, smem_u32(Bs + (k0 + 8 * (i & 1) + r) * kPB + n0));
+      mma_16816(acc, a[0], a[1], a[2], a[3], b[0], b[1]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sink_gradient(s, c, at[j], acc[j], m1v[j], m2v[j], pv[j]);
+    return;
+  }
+  // FP32 sums, one row after the other; thread n owns units n and n + 128
+  const AdamScale c(s);
+  auto sink = [&](int i, float gi) {
+    if (s.g) sink_gradient(s, c, i, gi, 0.f, 0.f, 0.f);
+    else sink_gradient(s, c, i, gi, s.m1[i], s.m2[i], s.p[i]);
+  };
+  if (blk == 144) {
+    __shared__ float s_dy[kMaxTrainRows], s_d[kMaxTrainRows];
+    for (int r = tid; r < B; r += 128) {
+      s_dy[r] = err[r];
+      s_d[r] = err[kMaxTrainRows + r];
+    }
+    __syncthreads();
+    const float w3a = s.p[kOffW3 + tid], w3b = s.p[kOffW3 + 128 + tid];
+    float gw0 = 0.f, gw1 = 0.f, gb0 = 0.f, gb1 = 0.f;
+#pragma unroll 16
+    for (int r = 0; r < B; ++r) {
+      const float dy = s_dy[r];
+      const float h0 = H2[(size_t)r * kHidden + tid], h1 = H2[(size_t)r * kHidden + 128 + tid];
+      gw0 = fmaf(dy, h0, gw0);
+      gw1 = fmaf(dy, h1, gw1);
+      gb0 = __fadd_rn(gb0, h0 > 0.f ? __fmul_rn(dy, w3a) : 0.f);
+      gb1 = __fadd_rn(gb1, h1 > 0.f ? __fmul_rn(dy, w3b) : 0.f);
+    }
+    sink(kOffW3 + tid, gw0);
+    sink(kOffW3 + 128 + tid, gw1);
+    sink(kOffB2 + tid, gb0);
+    sink(kOffB2 + 128 + tid, gb1);
+    if (tid == 0) {
+      float gb3 = 0.f, l = 0.f;
+      for (int r = 0; r < B; ++r) {
+        gb3 += s_dy[r];
+        l = fmaf(s_d[r], s_d[r], l);
+      }
+      sink(kOffB3, gb3);
+      *loss = l / (float)B;
+    }
+  } else {
+    float g0 = 0.f, g1 = 0.f;
+#pragma unroll 16
+    for (int r = 0; r < B; ++r) {
+      g0 += dZ1f[(size_t)r * kHidden + tid];
+      g1 += dZ1f[(size_t)r * kHidden + 128 + tid];
+    }
+    sink(kOffB1 + tid, g0);
+    sink(kOffB1 + 128 + tid, g1);
+  }
+}
 
 // BF16 copies of freshly written FP32 parameters.
-__global__ void cast_params_kernel(const float* __restrict__ p, bf16* __restrict__ w1b, bf16* __restrict__ w2b,
-                                   bf16* __restrict__ w2tb, bf16* __restrict__ w1u, bf16* __restrict__ w2u) {
+__global__ void cast_params_kernel(const float* __restrict__ p, bf16* __restrict__ w1u, bf16* __restrict__ w2u) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x)
-    store_bf16_copies(i, p[i], w1b, w2b, w2tb, w1u, w2u);
+    store_bf16_copies(i, p[i], w1u, w2u);
 }
 
-// Rows idx[0..B) of X (rows 0..B when idx is null) into Xs.
-__global__ void gather_rows_kernel(const bf16* __restrict__ X, const int* __restrict__ idx, int B,
-                                   bf16* __restrict__ Xs) {
-  const int n = B * kFeatures;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int r = i / kFeatures, c = i % kFeatures;
-    const int src = idx ? idx[r] : r;
-    Xs[i] = X[(long long)src * kFeatures + c];
-  }
+// FP32 features rounded to BF16 rows, four a thread.
+__global__ void cast_rows_kernel(const float4* __restrict__ x, uint2* __restrict__ out, int n4) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n4) return;
+  const float4 v = x[i];
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+  out[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
-
-int blocks_for(long long tiles) { return (int)((tiles + 3) / 4); }
 
 }  // namespace mlp
 
@@ -521,70 +712,27 @@ using namespace mlp;
 
 // ---- enqueue helpers the annealing engine uses ---------------------------------
 
-int mlp_forward(ggb_mlp* m, const bf16* X, int rows, float* y, cudaStream_t st, bool keep_z) {
+int mlp_forward(ggb_mlp* m, const bf16* X, int rows, float* y, cudaStream_t st) {
   if (rows % 16 || rows > m->max_rows) return core_fail(GGB_EINVAL, "mlp rows %d (max %d, multiple of 16)", rows, m->max_rows);
-  if (!keep_z) {
-    // inference: one fused launch on the tcgen05 tensor cores, the activations never leave the SM
-    forward_tc_kernel<<<(rows + tc::kRows - 1) / tc::kRows, tc::kThreads, tc::kSmem, st>>>(X, rows, m->W1u, m->W2u,
-                                                                                         m->p, y);
-    core_add_launches(1);
-    MCUDA(cudaGetLastError());
-    return GGB_OK;
-  }
-  EpiArgs e1 = {m->p + kOffB1, nullptr, m->H1, nullptr, nullptr};
-  gemm_tn_kernel<kEpiBiasReluBf16><<<blocks_for((long long)(rows / 16) * (kHidden / 8)), 128, 0, st>>>(
-      rows, kHidden, kFeatures, X, kFeatures, m->W1b, kFeatures, e1);
-  EpiArgs e2 = {m->p + kOffB2, nullptr, nullptr, m->H2, keep_z ? m->Z2 : nullptr};
-  gemm_tn_kernel<kEpiBiasReluF32><<<blocks_for((long long)(rows / 16) * (kHidden / 8)), 128, 0, st>>>(
-      rows, kHidden, kHidden, m->H1, kHidden, m->W2b, kHidden, e2);
-  head_kernel<<<(rows + 7) / 8, 256, 0, st>>>(m->H2, m->p + kOffW3, m->p + kOffB3, y, rows);
-  core_add_launches(3);
+  // one fused launch on the tcgen05 tensor cores, the activations never leave the SM
+  forward_tc_kernel<<<(rows + tc::kRows - 1) / tc::kRows, tc::kThreads, tc::kSmem, st>>>(X, rows, m->W1u, m->W2u, m->p,
+                                                                                       y);
+  core_add_launches(1);
   MCUDA(cudaGetLastError());
   return GGB_OK;
 }
 
-int mlp_backward(ggb_mlp* m, const bf16* Xs, const float* t, int B, cudaStream_t st) {
-  if (B % 16 || B > kMaxTrainRows || B > m->max_rows) return core_fail(GGB_EINVAL, "mlp training rows %d", B);
-  int rc = mlp_forward(m, Xs, B, m->y_train, st, true);
-  if (rc) return rc;
-  out_backward_kernel<<<1, kHidden, 0, st>>>(m->y_train, t, m->Z2, m->H2, m->p + kOffW3, B, m->dZ2, m->dZ2t, m->g,
-                                             m->loss);
-  transpose_bf16_kernel<<<64, 256, 0, st>>>(m->H1, m->H1t, B, kHidden);
-  // gW2[n][k] = sum_r dZ2[r][n] H1[r][k]:  A = dZ2t [256][B], Bt = H1t [256][B]
-  EpiArgs e2 = {nullptr, nullptr, nullptr, m->g + kOffW2, nullptr};
-  gemm_tn_kernel<kEpiF32><<<blocks_for((kHidden / 16) * (kHidden / 8)), 128, 0, st>>>(kHidden, kHidden, B, m->dZ2t, B,
-                                                                                   m->H1t, B, e2);
-  // dZ1[r][k] = (sum_n dZ2[r][n] W2[n][k]) * (H1[r][k] > 0):  A = dZ2 [B][256], Bt = W2t [256][256]
-  EpiArgs e3 = {nullptr, m->H1, m->dZ1, m->dZ1f, nullptr};
-  gemm_tn_kernel<kEpiMask><<<blocks_for((long long)(B / 16) * (kHidden / 8)), 128, 0, st>>>(B, kHidden, kHidden, m->dZ2,
-                                                                                        kHidden, m->W2tb, kHidden, e3);
-  col_sum_kernel<<<1, kHidden, 0, st>>>(m->dZ1f, B, kHidden, m->g + kOffB1);
-  transpose_bf16_kernel<<<64, 256, 0, st>>>(m->dZ1, m->dZ1t, B, kHidden);
-  transpose_bf16_kernel<<<16, 256, 0, st>>>(Xs, m->Xt, B, kFeatures);
-  // gW1[k][j] = sum_r dZ1[r][k] X[r][j]:  A = dZ1t [256][B], Bt = Xt [32][B]
-  EpiArgs e4 = {nullptr, nullptr, nullptr, m->g + kOffW1, nullptr};
-  gemm_tn_kernel<kEpiF32><<<blocks_for((kHidden / 16) * (kFeatures / 8)), 128, 0, st>>>(kHidden, kFeatures, B, m->dZ1t,
-                                                                                     B, m->Xt, B, e4);
-  core_add_launches(7);
-  MCUDA(cudaGetLastError());
-  return GGB_OK;
-}
-
-int mlp_adam(ggb_mlp* m, cudaStream_t st) {
-  adam_kernel<<<(kParams + 255) / 256, 256, 0, st>>>(m->p, m->g, m->m1, m->m2, m->step, m->hyper, m->W1b, m->W2b,
-                                                     m->W2tb, m->W1u, m->W2u);
-  adam_step_kernel<<<1, 1, 0, st>>>(m->step);
+int mlp_step(ggb_mlp* m, const bf16* X, const int* idx, const float* t, int B, bool adam, cudaStream_t st) {
+  if (B % 16 || B > kMaxTrainRows || (!idx && B > m->max_rows)) return core_fail(GGB_EINVAL, "mlp training rows %d", B);
+  train_rows_kernel<<<B / tr::kRows, tr::kThreads, tr::kSmem, st>>>(X, idx, t, B, m->W1u, m->W2u, m->p, m->H1, m->H2,
+                                                                   m->dZ2, m->dZ1, m->dZ1f, m->err, m->step,
+                                                                   adam ? 1 : 0);
+  const GradSink sink = {adam ? nullptr : m->g, m->p, m->m1, m->m2, m->step, m->hyper, m->W1u, m->W2u};
+  train_weights_kernel<<<kWeightBlocks, 128, 0, st>>>(X, idx, B, m->H1, m->H2, m->dZ2, m->dZ1, m->dZ1f, m->err, sink,
+                                                      m->loss);
   core_add_launches(2);
   MCUDA(cudaGetLastError());
   return GGB_OK;
-}
-
-int mlp_train_rows(ggb_mlp* m, const bf16* X, const int* idx, const float* t, int B, cudaStream_t st) {
-  gather_rows_kernel<<<8, 256, 0, st>>>(X, idx, B, m->Xs);
-  core_add_launches(1);
-  int rc = mlp_backward(m, m->Xs, t, B, st);
-  if (rc) return rc;
-  return mlp_adam(m, st);
 }
 
 size_t mlp_state_bytes() { return 3 * (size_t)kParams * sizeof(float) + sizeof(int); }
@@ -608,7 +756,7 @@ int mlp_load_state(ggb_mlp* m, const void* host) {
   MCUDA(cudaMemcpy(m->m1, h + pb, pb, cudaMemcpyHostToDevice));
   MCUDA(cudaMemcpy(m->m2, h + 2 * pb, pb, cudaMemcpyHostToDevice));
   MCUDA(cudaMemcpy(m->step, h + 3 * pb, sizeof(int), cudaMemcpyHostToDevice));
-  cast_params_kernel<<<64, 256>>>(m->p, m->W1b, m->W2b, m->W2tb, m->W1u, m->W2u);
+  cast_params_kernel<<<64, 256>>>(m->p, m->W1u, m->W2u);
   MCUDA(cudaGetLastError());
   MCUDA(cudaDeviceSynchronize());
   return GGB_OK;
@@ -654,18 +802,16 @@ int create(ggb_mlp* m, int max_rows, unsigned long long seed) {
   int rc;
   MCUDA(cudaFuncSetAttribute((const void*)forward_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)tc::kSmem));
-  const size_t R = (size_t)max_rows;
+  MCUDA(cudaFuncSetAttribute((const void*)train_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)tr::kSmem));
+  const size_t R = (size_t)max_rows, T = (size_t)kMaxTrainRows * kHidden;
   if ((rc = mdev(&m->p, kParams)) || (rc = mdev(&m->g, kParams)) || (rc = mdev(&m->m1, kParams)) ||
-      (rc = mdev(&m->m2, kParams)) || (rc = mdev(&m->step, 1)) || (rc = mdev(&m->W1b, (size_t)kOffB1)) ||
-      (rc = mdev(&m->W2b, (size_t)kHidden * kHidden)) || (rc = mdev(&m->W2tb, (size_t)kHidden * kHidden)) ||
-      (rc = mdev(&m->W1u, (size_t)kOffB1)) || (rc = mdev(&m->W2u, (size_t)kHidden * kHidden)) ||
-      (rc = mdev(&m->H1, R * kHidden)) || (rc = mdev(&m->H2, R * kHidden)) || (rc = mdev(&m->Z2, R * kHidden)) ||
-      (rc = mdev(&m->y_train, (size_t)kMaxTrainRows)) || (rc = mdev(&m->dZ2, (size_t)kMaxTrainRows * kHidden)) ||
-      (rc = mdev(&m->dZ2t, (size_t)kMaxTrainRows * kHidden)) || (rc = mdev(&m->H1t, (size_t)kMaxTrainRows * kHidden)) ||
-      (rc = mdev(&m->dZ1, (size_t)kMaxTrainRows * kHidden)) || (rc = mdev(&m->dZ1f, (size_t)kMaxTrainRows * kHidden)) ||
-      (rc = mdev(&m->dZ1t, (size_t)kMaxTrainRows * kHidden)) || (rc = mdev(&m->Xt, (size_t)kMaxTrainRows * kFeatures)) ||
-      (rc = mdev(&m->Xs, (size_t)kMaxTrainRows * kFeatures)) || (rc = mdev(&m->loss, 1)) ||
-      (rc = mdev(&m->X, R * kFeatures)) || (rc = mdev(&m->y, R)) || (rc = mdev(&m->t, (size_t)kMaxTrainRows)))
+      (rc = mdev(&m->m2, kParams)) || (rc = mdev(&m->step, 1)) || (rc = mdev(&m->W1u, (size_t)kOffB1)) ||
+      (rc = mdev(&m->W2u, (size_t)kHidden * kHidden)) || (rc = mdev(&m->H1, T)) || (rc = mdev(&m->H2, T)) ||
+      (rc = mdev(&m->dZ2, T)) || (rc = mdev(&m->dZ1, T)) || (rc = mdev(&m->dZ1f, T)) ||
+      (rc = mdev(&m->err, 2 * (size_t)kMaxTrainRows)) || (rc = mdev(&m->loss, 1)) ||
+      (rc = mdev(&m->X, R * kFeatures)) || (rc = mdev(&m->xf, R * kFeatures)) || (rc = mdev(&m->y, R)) ||
+      (rc = mdev(&m->t, (size_t)kMaxTrainRows)))
     return rc;
   std::vector<float> p;
   init_params(p, seed);
@@ -674,20 +820,23 @@ int create(ggb_mlp* m, int max_rows, unsigned long long seed) {
 
 void destroy(ggb_mlp* m) {
   if (!m) return;
-  for (void* q : {(void*)m->p, (void*)m->g, (void*)m->m1, (void*)m->m2, (void*)m->step, (void*)m->W1b, (void*)m->W2b,
-                  (void*)m->W2tb, (void*)m->W1u, (void*)m->W2u, (void*)m->H1, (void*)m->H2, (void*)m->Z2, (void*)m->y_train, (void*)m->dZ2,
-                  (void*)m->dZ2t, (void*)m->H1t, (void*)m->dZ1, (void*)m->dZ1f, (void*)m->dZ1t, (void*)m->Xt,
-                  (void*)m->Xs, (void*)m->loss, (void*)m->X, (void*)m->y, (void*)m->t})
+  for (void* q : {(void*)m->p, (void*)m->g, (void*)m->m1, (void*)m->m2, (void*)m->step, (void*)m->W1u, (void*)m->W2u,
+                  (void*)m->H1, (void*)m->H2, (void*)m->dZ2, (void*)m->dZ1, (void*)m->dZ1f, (void*)m->err,
+                  (void*)m->loss, (void*)m->X, (void*)m->xf, (void*)m->y, (void*)m->t})
     cudaFree(q);
   cudaGetLastError();
   delete m;
 }
 
-// Host FP32 features -> device BF16 rows of m->X.
+// Host FP32 features -> device BF16 rows of m->X (rounded on the device; on the
+// host the rounding of 4096 rows took longer than the forward).
 int upload_x(ggb_mlp* m, const float* x, int rows) {
-  std::vector<bf16> xb((size_t)rows * ggb::mlp::kFeatures);
-  for (size_t i = 0; i < xb.size(); ++i) xb[i] = __float2bfloat16_rn(x[i]);
-  MCUDA(cudaMemcpy(m->X, xb.data(), xb.size() * sizeof(bf16), cudaMemcpyHostToDevice));
+  const int n4 = rows * ggb::mlp::kFeatures / 4;
+  MCUDA(cudaMemcpy(m->xf, x, (size_t)rows * ggb::mlp::kFeatures * sizeof(float), cudaMemcpyHostToDevice));
+  ggb::mlp::cast_rows_kernel<<<(n4 + 255) / 256, 256>>>(reinterpret_cast<const float4*>(m->xf),
+                                                       reinterpret_cast<uint2*>(m->X), n4);
+  ggb::core_add_launches(1);
+  MCUDA(cudaGetLastError());
   return GGB_OK;
 }
 
@@ -720,7 +869,7 @@ int ggb_mlp_set_params(ggb_mlp* m, const float* params) {
   MCUDA(cudaMemset(m->m1, 0, kParams * sizeof(float)));
   MCUDA(cudaMemset(m->m2, 0, kParams * sizeof(float)));
   MCUDA(cudaMemset(m->step, 0, sizeof(int)));
-  cast_params_kernel<<<64, 256>>>(m->p, m->W1b, m->W2b, m->W2tb, m->W1u, m->W2u);
+  cast_params_kernel<<<64, 256>>>(m->p, m->W1u, m->W2u);
   MCUDA(cudaGetLastError());
   MCUDA(cudaDeviceSynchronize());
   return GGB_OK;
@@ -745,7 +894,7 @@ int ggb_mlp_forward_host(ggb_mlp* m, const float* x, int rows, float* y) {
   if (rows <= 0 || rows % 16 || rows > m->max_rows) return core_fail(GGB_EINVAL, "rows must be a multiple of 16 up to max_rows");
   int rc = upload_x(m, x, rows);
   if (rc) return rc;
-  rc = ggb::mlp_forward(m, m->X, rows, m->y, nullptr, false);
+  rc = ggb::mlp_forward(m, m->X, rows, m->y, nullptr);
   if (rc) return rc;
   MCUDA(cudaMemcpy(y, m->y, (size_t)rows * sizeof(float), cudaMemcpyDeviceToHost));
   return GGB_OK;
@@ -764,10 +913,10 @@ int ggb_mlp_time_forward(ggb_mlp* m, const float* x, int rows, int reps, double*
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
   float t = 0.f;
   if (e == cudaSuccess) {
-    rc = ggb::mlp_forward(m, m->X, rows, m->y, st, false);   // warm-up
+    rc = ggb::mlp_forward(m, m->X, rows, m->y, st);   // warm-up
     if (rc == GGB_OK) e = cudaEventRecord(e0, st);
     for (int i = 0; i < reps && rc == GGB_OK && e == cudaSuccess; ++i)
-      rc = ggb::mlp_forward(m, m->X, rows, m->y, st, false);
+      rc = ggb::mlp_forward(m, m->X, rows, m->y, st);
     if (rc == GGB_OK && e == cudaSuccess) e = cudaEventRecord(e1, st);
     if (rc == GGB_OK && e == cudaSuccess) e = cudaEventSynchronize(e1);
     if (rc == GGB_OK && e == cudaSuccess) e = cudaEventElapsedTime(&t, e0, e1);
@@ -791,7 +940,7 @@ int ggb_mlp_grads_host(ggb_mlp* m, const float* x, const float* t, int rows, flo
   int rc = upload_x(m, x, rows);
   if (rc) return rc;
   MCUDA(cudaMemcpy(m->t, t, (size_t)rows * sizeof(float), cudaMemcpyHostToDevice));
-  rc = ggb::mlp_backward(m, m->X, m->t, rows, nullptr);
+  rc = ggb::mlp_step(m, m->X, nullptr, m->t, rows, false, nullptr);
   if (rc) return rc;
   MCUDA(cudaDeviceSynchronize());
   MCUDA(cudaMemcpy(grads, m->g, ggb::mlp::kParams * sizeof(float), cudaMemcpyDeviceToHost));
@@ -807,9 +956,7 @@ int ggb_mlp_train_host(ggb_mlp* m, const float* x, const float* t, int rows, int
   if (rc) return rc;
   MCUDA(cudaMemcpy(m->t, t, (size_t)rows * sizeof(float), cudaMemcpyHostToDevice));
   for (int s = 0; s < steps; ++s) {
-    rc = ggb::mlp_backward(m, m->X, m->t, rows, nullptr);
-    if (rc) return rc;
-    rc = ggb::mlp_adam(m, nullptr);
+    rc = ggb::mlp_step(m, m->X, nullptr, m->t, rows, true, nullptr);
     if (rc) return rc;
   }
   MCUDA(cudaDeviceSynchronize());

@@ -36,44 +36,33 @@ struct ggb_mlp {
   float* m1 = nullptr;         // Adam moments
   float* m2 = nullptr;
   int* step = nullptr;         // Adam step count (device)
-  __nv_bfloat16* W1b = nullptr;    // [256][32]
-  __nv_bfloat16* W2b = nullptr;    // [256][256]
-  __nv_bfloat16* W2tb = nullptr;   // W2 transposed
-  // W1 and W2 in the tensor cores' shared-memory operand layout (K-major,
-  // no swizzle: 8-row x 16-byte core matrices), staged by one bulk copy each
+  // W1 and W2 as BF16 in the tensor cores' shared-memory operand layout
+  // (K-major, no swizzle: 8-row x 16-byte core matrices), staged by bulk copies
   __nv_bfloat16* W1u = nullptr;    // [256][32] tiled
   __nv_bfloat16* W2u = nullptr;    // [256][256] tiled
-  // activations and workspaces
-  __nv_bfloat16* H1 = nullptr;     // [max_rows][256]
-  float* H2 = nullptr;             // [max_rows][256]
-  float* Z2 = nullptr;             // [max_rows][256]
-  float* y_train = nullptr;        // [kMaxTrainRows]
-  __nv_bfloat16* dZ2 = nullptr;    // [kMaxTrainRows][256]
-  __nv_bfloat16* dZ2t = nullptr;
-  __nv_bfloat16* H1t = nullptr;
+  // what a training step hands from its row pass to its weight pass, [kMaxTrainRows][256]
+  __nv_bfloat16* H1 = nullptr;
+  __nv_bfloat16* dZ2 = nullptr;
   __nv_bfloat16* dZ1 = nullptr;
+  float* H2 = nullptr;
   float* dZ1f = nullptr;
-  __nv_bfloat16* dZ1t = nullptr;
-  __nv_bfloat16* Xt = nullptr;     // [32][kMaxTrainRows]
-  __nv_bfloat16* Xs = nullptr;     // gathered training rows [kMaxTrainRows][32]
+  float* err = nullptr;        // [2][kMaxTrainRows]: dy, y - t
   float* loss = nullptr;
   // host-entry staging
   __nv_bfloat16* X = nullptr;      // [max_rows][32]
+  float* xf = nullptr;             // [max_rows][32] as the caller gave them
   float* y = nullptr;              // [max_rows]
   float* t = nullptr;              // [kMaxTrainRows]
 };
 
 namespace ggb {
 
-// y[0..rows) = network(X rows); rows % 16 == 0.  keep_z keeps the second
-// layer's pre-activations for a backward pass.
-int mlp_forward(ggb_mlp* m, const __nv_bfloat16* X, int rows, float* y, cudaStream_t st, bool keep_z);
-// Gradients of the mean squared error over B rows (B % 16 == 0, B <= 256).
-int mlp_backward(ggb_mlp* m, const __nv_bfloat16* Xs, const float* t, int B, cudaStream_t st);
-// One Adam step with the last gradients.
-int mlp_adam(ggb_mlp* m, cudaStream_t st);
-// Gathers rows idx[0..B) of X, then backward + Adam on them with targets t.
-int mlp_train_rows(ggb_mlp* m, const __nv_bfloat16* X, const int* idx, const float* t, int B, cudaStream_t st);
+// y[0..rows) = network(X rows); rows % 16 == 0.
+int mlp_forward(ggb_mlp* m, const __nv_bfloat16* X, int rows, float* y, cudaStream_t st);
+// Loss and gradients of the mean squared error over B rows (B % 16 == 0,
+// B <= 256) -- rows idx[0..B) of X, or 0..B-1 when idx is null -- into m->loss
+// and m->g; with adam, one Adam step on them instead of writing m->g.
+int mlp_step(ggb_mlp* m, const __nv_bfloat16* X, const int* idx, const float* t, int B, bool adam, cudaStream_t st);
 // The training state (FP32 parameters, both Adam moments, the Adam step) as
 // host bytes: its size, a copy out and a copy in (which also refreshes every
 // BF16 copy of the weights).  Synchronous.

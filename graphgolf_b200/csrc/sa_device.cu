@@ -982,7 +982,7 @@ int enqueue_step(ggb_sa* a, cudaStream_t st) {
   if (a->learned) {
     features_kernel<<<(G + 127) / 128, 128, 0, st>>>(s, a->d_swaps, G, a->d_stats, a->d_levels, a->d_winlev,
                                                      a->level_cap, a->d_X);
-    int rc = ggb::mlp_forward(a->mlp, a->d_X, G, a->d_scores, st, false);
+    int rc = ggb::mlp_forward(a->mlp, a->d_X, G, a->d_scores, st);
     if (rc) return rc;
     select_kernel<<<1, 1024, 0, st>>>(s, a->d_swaps, a->d_scores, G, a->K, a->n_rand, a->d_sel, a->d_rank,
                                       a->d_rank_key);
@@ -1033,7 +1033,7 @@ int enqueue_step(ggb_sa* a, cudaStream_t st) {
                                                                    a->d_pred, a->comp ? a->C : 0);
   launches += 1;
   if (a->learned) {
-    rc = ggb::mlp_train_rows(a->mlp, a->d_X, a->d_sel, a->d_labels, a->K, st);
+    rc = ggb::mlp_step(a->mlp, a->d_X, a->d_sel, a->d_labels, a->K, true, st);
     if (rc) return rc;
   }
   if (a->has_base) {
