@@ -496,10 +496,12 @@ int ggb::batch_enqueue(ggb_batch* b, cudaStream_t st) {
   for (const auto& l : b->slices) {
     if (l.words == 1)
       ggb::slice_batch_kernel<1><<<l.items, l.threads, l.smem, st>>>(b->d_graphs, b->d_items + l.first, b->d_records,
-                                                                    b->d_out, b->stop, b->sticky);
+                                                                    b->d_out, b->patch_base, b->patch, b->stop,
+                                                                    b->sticky);
     else
       ggb::slice_batch_kernel<2><<<l.items, l.threads, l.smem, st>>>(b->d_graphs, b->d_items + l.first, b->d_records,
-                                                                    b->d_out, b->stop, b->sticky);
+                                                                    b->d_out, b->patch_base, b->patch, b->stop,
+                                                                    b->sticky);
     BCUDA(cudaGetLastError());
   }
   return GGB_OK;

@@ -493,6 +493,7 @@ ggb::SliceArgs slice_args(int N, int d, int n_src1, int split, int ac, int group
   a.adj = nullptr;
   a.adj16 = nullptr;
   a.deg = nullptr;
+  a.patch = nullptr;
   a.ctrl = g.d_sctrl;
   a.out = g.h_sout;
   a.N = N;

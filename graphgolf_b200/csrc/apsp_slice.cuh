@@ -24,6 +24,7 @@ struct SliceArgs {
   const int* adj;            // [N][d] ids, or null when adj16 is given
   const uint16_t* adj16;     // [N][d] 16-bit ids
   const int* deg;            // entries of row v that count, in [0, d] (null: all)
+  const Swap* patch;         // the graph is adj with this swap applied when it is valid (null: adj itself)
   ApspCtrl* ctrl;            // all zero between launches (the last CTA clears it)
   ApspCtrl* out;             // the result record (pinned host memory), written by the last CTA
   int N, d, pairs, np;       // np = N rounded up to 32
@@ -179,6 +180,14 @@ __device__ __forceinline__ SliceTotals slice_windows(const SliceArgs& a, int t0,
     if (bad) set_error(a.ctrl, kErrAdj, v);
   }
   __syncthreads();
+  if (a.patch && a.patch->valid) {
+    // row x[q]'s entry pos[q] becomes x[q ^ 2]; the four rows are distinct
+    if (tid < 4) {
+      uint16_t* e = reinterpret_cast<uint16_t*>(s_adj + (a.patch->pos[tid] >> 1) * np + a.patch->x[tid]);
+      e[a.patch->pos[tid] & 1] = (uint16_t)a.patch->x[tid ^ 2];
+    }
+    __syncthreads();
+  }
 
   SliceTotals r;
   unsigned g = 0;                      // levels run so far: the rotation of s_cnt
@@ -257,17 +266,21 @@ __global__ void __launch_bounds__(1024, 1) slice_kernel(const SliceArgs a) {
 // ---- many small graphs, one launch ---------------------------------------------------
 // CTA i takes the windows items[i] of one graph of a batch (see BatchGraph);
 // each graph has a record of its own, and the last of its CTAs writes its
-// BatchOut.  Nothing to clear before the launch.
+// BatchOut.  Nothing to clear before the launch.  With base, graph i is base
+// with patch[i] applied (an annealer's candidates, never written out).
 template <int WORDS>
 __global__ void __launch_bounds__(1024, 1) slice_batch_kernel(const BatchGraph* __restrict__ graphs,
                                                               const SliceItem* __restrict__ items,
                                                               ApspCtrl* __restrict__ records, BatchOut* __restrict__ out,
-                                                              const int* stop, int* sticky) {
+                                                              const int* __restrict__ base,
+                                                              const Swap* __restrict__ patch, const int* stop,
+                                                              int* sticky) {
   if (stop && ld_volatile_i32(stop) != 0) return;   // written before the launch: the same in every CTA
   const SliceItem it = items[blockIdx.x];
   const BatchGraph gr = graphs[it.graph];
   SliceArgs a;
-  a.adj = gr.adj;
+  a.adj = base ? base : gr.adj;
+  a.patch = base ? patch + it.graph : nullptr;
   a.adj16 = nullptr;
   a.deg = nullptr;
   a.ctrl = records + it.graph;

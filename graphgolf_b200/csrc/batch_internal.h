@@ -70,6 +70,11 @@ struct ggb_batch {
   cudaGraphExec_t exec = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
   bool pending = false;
+  // Graph i is patch_base with patch[i] applied instead of its own adjacency
+  // (device; only while every graph is on slices, see all_slices).
+  const int* patch_base = nullptr;
+  const ggb::Swap* patch = nullptr;
+  bool all_slices() const { return split && l_teams == 0 && n_teams == 0 && !slice_items.empty(); }
   const int* stop = nullptr;         // device flag: the launch does nothing while it is non-zero
   int* sticky = nullptr;             // device flag: first error code of any launch (set, never cleared)
 };

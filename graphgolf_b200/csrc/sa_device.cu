@@ -110,10 +110,14 @@ __device__ __forceinline__ int below(unsigned long long h, int n) {
   return (int)(((h >> 32) * (unsigned long long)(unsigned)n) >> 32);
 }
 
+// The first place of x in a row, or -1.  Every entry is read (no early exit), so
+// that the loads are in flight together.
 __device__ __forceinline__ int find_in_row(const int* row, int d, int x) {
-  for (int j = 0; j < d; ++j)
-    if (row[j] == x) return j;
-  return -1;
+  int p = -1;
+#pragma unroll 8
+  for (int j = d - 1; j >= 0; --j)
+    if (row[j] == x) p = j;
+  return p;
 }
 
 // ---- gen: candidate swaps ------------------------------------------------------
@@ -169,6 +173,45 @@ __device__ bool gen_orbit_move(const State* s, unsigned long long h, Swap& w) {
   return true;
 }
 
+// Attempt `attempt` of proposal k in this step; false when it draws no valid move.
+__device__ bool gen_attempt(const State* s, int k, int attempt, Swap& w) {
+  const int lines = s->lines, d = s->d;
+  const int* E = s->edges;
+  const int* A = s->adj;
+  const unsigned long long h = draw(s->seed, (unsigned long long)s->step, (unsigned long long)k,
+                                    (unsigned long long)attempt);
+  w.kind = 0;
+  if (s->groups > 1) return gen_orbit_move(s, h, w);
+  const int i = below(h, lines), j = below(h << 32, lines);
+  if (i == j) return false;
+  const int r = (int)(mix64(h) & 1);
+  const int a = E[2 * i], b = E[2 * i + 1], c = E[2 * j], e = E[2 * j + 1];
+  const int x0 = a, x1 = b, x2 = r ? e : c, x3 = r ? c : e;
+  if (x0 == x2 || x1 == x3) return false;
+  // grid graphs: both new edges within the length limit (grid/sa.c:196-201)
+  if (s->grid_length > 0 && (manhattan(x0, x2, s->grid_height) > s->grid_length ||
+                             manhattan(x1, x3, s->grid_height) > s->grid_length))
+    return false;
+  const int* r0 = A + (long long)x0 * d;
+  const int* r1 = A + (long long)x1 * d;
+  const int* r2 = A + (long long)x2 * d;
+  const int* r3 = A + (long long)x3 * d;
+  const int n0 = find_in_row(r0, d, x2), n1 = find_in_row(r1, d, x3);
+  const int p0 = find_in_row(r0, d, x1), p1 = find_in_row(r1, d, x0);
+  const int p2 = find_in_row(r2, d, x3), p3 = find_in_row(r3, d, x2);
+  if (n0 >= 0 || n1 >= 0) return false;
+  if (p0 < 0 || p1 < 0 || p2 < 0 || p3 < 0) return false;
+  w.line[0] = i;
+  w.line[1] = j;
+  w.x[0] = x0; w.x[1] = x1; w.x[2] = x2; w.x[3] = x3;
+  w.pos[0] = p0; w.pos[1] = p1; w.pos[2] = p2; w.pos[3] = p3;
+  return true;
+}
+
+// a length limit rejects most random pairs of lines (both new edges must be
+// short): draw more of them; the length test comes before any row scan
+__device__ __forceinline__ int gen_attempts(const State* s) { return s->grid_length > 0 ? 1024 : 64; }
+
 __global__ void gen_kernel(const State* __restrict__ s, Swap* __restrict__ out, int G) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= G) return;
@@ -176,43 +219,31 @@ __global__ void gen_kernel(const State* __restrict__ s, Swap* __restrict__ out, 
   w.valid = 0;
   w.kind = 0;
   if (!s->done) {
-    const int lines = s->lines, d = s->d;
-    const int* __restrict__ E = s->edges;
-    const int* __restrict__ A = s->adj;
-    const unsigned long long seed = s->seed, step = (unsigned long long)s->step;
-    // a length limit rejects most random pairs of lines (both new edges must be
-    // short): draw more of them; the length test comes before any row scan
-    const int attempts = s->grid_length > 0 ? 1024 : 64;
-    for (int attempt = 0; attempt < attempts && !w.valid; ++attempt) {
-      const unsigned long long h = draw(seed, step, (unsigned long long)k, (unsigned long long)attempt);
-      if (s->groups > 1) {
-        if (gen_orbit_move(s, h, w)) w.valid = 1;
-        continue;
-      }
-      const int i = below(h, lines), j = below(h << 32, lines);
-      if (i == j) continue;
-      const int r = (int)(mix64(h) & 1);
-      const int a = E[2 * i], b = E[2 * i + 1], c = E[2 * j], e = E[2 * j + 1];
-      const int x0 = a, x1 = b, x2 = r ? e : c, x3 = r ? c : e;
-      if (x0 == x2 || x1 == x3) continue;
-      // grid graphs: both new edges within the length limit (grid/sa.c:196-201)
-      if (s->grid_length > 0 && (manhattan(x0, x2, s->grid_height) > s->grid_length ||
-                                 manhattan(x1, x3, s->grid_height) > s->grid_length))
-        continue;
-      const int* r0 = A + (long long)x0 * d;
-      const int* r1 = A + (long long)x1 * d;
-      if (find_in_row(r0, d, x2) >= 0 || find_in_row(r1, d, x3) >= 0) continue;
-      const int p0 = find_in_row(r0, d, x1), p1 = find_in_row(r1, d, x0);
-      const int p2 = find_in_row(A + (long long)x2 * d, d, x3), p3 = find_in_row(A + (long long)x3 * d, d, x2);
-      if (p0 < 0 || p1 < 0 || p2 < 0 || p3 < 0) continue;
-      w.line[0] = i;
-      w.line[1] = j;
-      w.x[0] = x0; w.x[1] = x1; w.x[2] = x2; w.x[3] = x3;
-      w.pos[0] = p0; w.pos[1] = p1; w.pos[2] = p2; w.pos[3] = p3;
-      w.valid = 1;
-    }
+    const int attempts = gen_attempts(s);
+    for (int attempt = 0; attempt < attempts && !w.valid; ++attempt)
+      if (gen_attempt(s, k, attempt, w)) w.valid = 1;
   }
   out[k] = w;
+}
+
+// Proposal 0 by one warp, a lane an attempt; the first valid attempt counts, as
+// in gen_kernel.
+__device__ void gen_one(const State* s, Swap* out) {
+  const int lane = threadIdx.x & 31, attempts = gen_attempts(s);
+  for (int a0 = 0; a0 < attempts; a0 += 32) {
+    Swap w;
+    w.valid = a0 + lane < attempts && gen_attempt(s, 0, a0 + lane, w) ? 1 : 0;
+    const unsigned m = __ballot_sync(0xffffffffu, w.valid != 0);
+    if (!m) continue;
+    if (lane == __ffs(m) - 1) *out = w;
+    return;
+  }
+  if (lane == 0) {
+    Swap w;
+    w.valid = 0;
+    w.kind = 0;
+    *out = w;
+  }
 }
 
 // ---- materialize: candidate adjacencies into the batch slots ---------------------
@@ -325,19 +356,6 @@ __device__ __forceinline__ int move_classes(const State* s, const Swap& w, int* 
   return 4;
 }
 
-__device__ __forceinline__ bool classes_free(const unsigned* vmark, const int* c, int n) {
-  bool f = true;
-  for (int q = 0; q < n; ++q) f &= !((vmark[c[q] >> 5] >> (c[q] & 31)) & 1u);
-  return f;
-}
-
-__device__ __forceinline__ void classes_set(unsigned* vmark, const int* c, int n, bool on) {
-  for (int q = 0; q < n; ++q) {
-    if (on) vmark[c[q] >> 5] |= 1u << (c[q] & 31);
-    else vmark[c[q] >> 5] = 0u;
-  }
-}
-
 // Orbit moves of the candidates: slot k (block k) = the current adjacency,
 // copied by materialize_kernel, with candidate sel[k]'s move applied.
 __global__ void patch_orbit_kernel(State* __restrict__ s, const Swap* __restrict__ sw, const int* __restrict__ sel,
@@ -381,6 +399,55 @@ __device__ __forceinline__ bool key_less(const Key& a, const Key& b) {
   return a.diam < b.diam || (a.diam == b.diam && a.total < b.total);
 }
 
+// Walks a ranking best first and keeps, up to `limit`, the moves whose vertex
+// classes none of the kept ones touch; one warp, 32 of the ranking at a time.
+// get(r, w): 0 the ranking ends at r, 1 r is passed over, 2 r is the move w.
+// vmark (a bit per class) is all zero before and after.  Returns how many moves
+// it wrote to out, in order.
+template <typename Get>
+__device__ int greedy_disjoint(const State* s, unsigned* vmark, int n, int limit, Swap* out, Get get) {
+  const int lane = threadIdx.x & 31;
+  const unsigned all = 0xffffffffu;
+  int m = 0;
+  for (int r0 = 0; r0 < n && m < limit; r0 += 32) {
+    Swap w;
+    int c[4] = {-1, -1, -1, -1};
+    const int what = r0 + lane < n ? get(r0 + lane, w) : 0;
+    const unsigned ends = __ballot_sync(all, what == 0);
+    bool free = what == 2 && (!ends || lane < __ffs(ends) - 1);
+    if (free) {
+      const int nc = move_classes(s, w, c);
+      for (int q = 0; q < nc; ++q) free &= !((__ldcg(vmark + (c[q] >> 5)) >> (c[q] & 31)) & 1u);
+    }
+    unsigned left = __ballot_sync(all, free), kept = 0u;
+    while (left && m + __popc(kept) < limit) {
+      const int k = __ffs(left) - 1;
+      kept |= 1u << k;
+      bool hit = false;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int x = __shfl_sync(all, c[q], k);
+        hit |= x >= 0 && (c[0] == x || c[1] == x || c[2] == x || c[3] == x);
+      }
+      left = __ballot_sync(all, free && !hit) & left & ~((2u << k) - 1u);
+    }
+    if ((kept >> lane) & 1u) {
+      out[m + __popc(kept & ((1u << lane) - 1u))] = w;
+      for (int q = 0; q < 4; ++q)
+        if (c[q] >= 0) atomicOr(vmark + (c[q] >> 5), 1u << (c[q] & 31));
+    }
+    m += __popc(kept);
+    __syncwarp();
+    if (ends) break;
+  }
+  for (int i = lane; i < m; i += 32) {
+    int c[4];
+    const int nc = move_classes(s, out[i], c);
+    for (int q = 0; q < nc; ++q) __stcg(vmark + (c[q] >> 5), 0u);
+  }
+  return m;
+}
+
 // ---- compose: rank the candidates, build the composite -----------------------------
 // One block of kComposeThreads threads, K <= kComposeThreads.
 constexpr int kComposeThreads = 256;
@@ -406,29 +473,19 @@ __global__ void __launch_bounds__(kComposeThreads) compose_kernel(State* __restr
     s_order[rank] = k;
   }
   __syncthreads();
-  if (k != 0) return;
-  s->prev_total = s->cur_total;
-  s->best_k = s_order[0];
+  if (k >= 32) return;
   const Key cur = {s->cur_diam, s->cur_total};
-  int m = 0;
-  for (int r = 0; r < K && m < compose_max; ++r) {
+  const int m = greedy_disjoint(s, vmark, K, compose_max, comp, [&](int r, Swap& w) -> int {
     const int c = s_order[r];
-    const Key kc = s_keys[c];
-    if (!key_less(kc, cur)) break;   // sorted: nothing further improves
-    const Swap w = sw[sel ? sel[c] : c];
-    if (!w.valid) continue;
-    int cl[4];
-    const int nc = move_classes(s, w, cl);
-    if (!classes_free(vmark, cl, nc)) continue;
-    classes_set(vmark, cl, nc, true);
-    comp[m++] = w;
+    if (!key_less(s_keys[c], cur)) return 0;   // sorted: nothing further improves
+    w = sw[sel ? sel[c] : c];
+    return w.valid ? 2 : 1;
+  });
+  if (k == 0) {
+    s->prev_total = s->cur_total;
+    s->best_k = s_order[0];
+    s->n_comp = m;
   }
-  for (int i = 0; i < m; ++i) {
-    int cl[4];
-    const int nc = move_classes(s, comp[i], cl);
-    classes_set(vmark, cl, nc, false);
-  }
-  s->n_comp = m;
 }
 
 // Size of predicted composite c: the first n_pred >> c swaps of the list.
@@ -443,11 +500,15 @@ __device__ __forceinline__ int pred_size(int n_pred, int c) { return n_pred >> c
 // write the training labels of this step.
 // comp_out (when there is a composite batch): [0] the exact composite,
 // [1 + c] predicted composite c.
-__global__ void decide_kernel(State* __restrict__ s, const Swap* __restrict__ sw, const int* __restrict__ sel,
-                              const BatchOut* __restrict__ out, int K, const Swap* __restrict__ comp,
-                              const BatchOut* __restrict__ comp_out, float* __restrict__ labels,
-                              const Swap* __restrict__ pred, int C) {
-  if (s->done) return;
+
+// One block; thread 0 decides, the block applies the chosen moves (they touch
+// disjoint rows).  Every thread calls it.
+__device__ __forceinline__ void decide_step(State* __restrict__ s, const Swap* __restrict__ sw,
+                                            const int* __restrict__ sel, const BatchOut* __restrict__ out, int K,
+                                            const Swap* __restrict__ comp, const BatchOut* __restrict__ comp_out,
+                                            float* __restrict__ labels, const Swap* __restrict__ pred, int C) {
+  __shared__ const Swap* s_moves;
+  __shared__ int s_n;
   const int N = s->N;
   const int k = threadIdx.x;
   if (k < K && !out[k].done) atomicAdd(reinterpret_cast<unsigned long long*>(&s->unevaluated), 1ULL);
@@ -460,74 +521,112 @@ __global__ void decide_kernel(State* __restrict__ s, const Swap* __restrict__ sw
     }
     labels[k] = lab;
   }
-  if (k != 0) return;
-  const Key cur = {s->cur_diam, s->cur_total};
-  const int bk = s->best_k;
-  Key cand = cand_key(sw, sel, out, bk, N);
-  bool use_comp = false;
-  int use_pred = 0;   // swaps of the chosen predicted composite (0: none)
-  if (comp_out && s->n_comp >= 2) {
-    const Key kc = key_of(comp_out[0], N);
-    if (key_less(kc, cand)) {
-      cand = kc;
-      use_comp = true;
-    }
-  }
-  for (int c = 0; c < C && comp_out; ++c) {
-    const int m = pred_size(s->n_pred, c);
-    if (m < 1) break;
-    const Key kp = key_of(comp_out[1 + c], N);
-    if (key_less(kp, cand)) {
-      cand = kp;
-      use_comp = false;
-      use_pred = m;
-    }
-  }
-  bool acc = false;
-  if (cand.diam != INT_MAX) {
-    if (cand.diam < cur.diam) {
-      acc = true;
-    } else if (cand.diam == cur.diam) {
-      if (cand.total <= cur.total) {
-        acc = true;
-      } else if (!s->hill) {
-        const double diff = (double)(cur.total - cand.total) / (double)s->groups;
-        const unsigned long long h = draw(s->seed ^ 0x5bd1e995ULL, (unsigned long long)s->step, 0x0dec1deULL, 7);
-        const double u = ((double)(h >> 11) + 1.0) / (9007199254740992.0 + 2.0);
-        acc = exp(diff / s->temp) > u;
+  if (k == 0) {
+    s_n = 0;
+    const Key cur = {s->cur_diam, s->cur_total};
+    const int bk = s->best_k;
+    Key cand = cand_key(sw, sel, out, bk, N);
+    bool use_comp = false;
+    int use_pred = 0;   // swaps of the chosen predicted composite (0: none)
+    if (comp_out && s->n_comp >= 2) {
+      const Key kc = key_of(comp_out[0], N);
+      if (key_less(kc, cand)) {
+        cand = kc;
+        use_comp = true;
       }
     }
-  }
-  s->evals += K + C + (comp_out ? 1 : 0);
-  if (acc) {
-    bool ok = true;
-    if (use_pred) {
-      for (int i = 0; i < use_pred; ++i) ok &= apply_move(s, s->adj, s->edges, pred[i]);
-      s->multi_accepts += 1;
-      s->pred_accepts += 1;
-      s->moved_swaps += use_pred;
-    } else if (use_comp) {
-      for (int i = 0; i < s->n_comp; ++i) ok &= apply_move(s, s->adj, s->edges, comp[i]);
-      s->multi_accepts += 1;
-      s->moved_swaps += s->n_comp;
-    } else {
-      ok &= apply_move(s, s->adj, s->edges, sw[sel ? sel[bk] : bk]);
-      s->moved_swaps += 1;
+    for (int c = 0; c < C && comp_out; ++c) {
+      const int m = pred_size(s->n_pred, c);
+      if (m < 1) break;
+      const Key kp = key_of(comp_out[1 + c], N);
+      if (key_less(kp, cand)) {
+        cand = kp;
+        use_comp = false;
+        use_pred = m;
+      }
     }
-    if (!ok) s->move_error = 1;
-    s->accepts += 1;
-    s->cur_diam = cand.diam;
-    s->cur_total = cand.total;
-    if (cand.diam < s->best_diam || (cand.diam == s->best_diam && cand.total < s->best_total)) {
-      s->best_diam = cand.diam;
-      s->best_total = cand.total;
-      s->best_step = s->step;
+    bool acc = false;
+    if (cand.diam != INT_MAX) {
+      if (cand.diam < cur.diam) {
+        acc = true;
+      } else if (cand.diam == cur.diam) {
+        if (cand.total <= cur.total) {
+          acc = true;
+        } else if (!s->hill) {
+          const double diff = (double)(cur.total - cand.total) / (double)s->groups;
+          const unsigned long long h = draw(s->seed ^ 0x5bd1e995ULL, (unsigned long long)s->step, 0x0dec1deULL, 7);
+          const double u = ((double)(h >> 11) + 1.0) / (9007199254740992.0 + 2.0);
+          acc = exp(diff / s->temp) > u;
+        }
+      }
     }
+    s->evals += K + C + (comp_out ? 1 : 0);
+    if (acc) {
+      if (use_pred) {
+        s_moves = pred;
+        s_n = use_pred;
+        s->multi_accepts += 1;
+        s->pred_accepts += 1;
+      } else if (use_comp) {
+        s_moves = comp;
+        s_n = s->n_comp;
+        s->multi_accepts += 1;
+      } else {
+        s_moves = sw + (sel ? sel[bk] : bk);
+        s_n = 1;
+      }
+      s->moved_swaps += s_n;
+      s->accepts += 1;
+      s->cur_diam = cand.diam;
+      s->cur_total = cand.total;
+      if (cand.diam < s->best_diam || (cand.diam == s->best_diam && cand.total < s->best_total)) {
+        s->best_diam = cand.diam;
+        s->best_total = cand.total;
+        s->best_step = s->step;
+      }
+    }
+    s->accepted = acc ? 1 : 0;
+    if (s->stop_on_target && s->cur_diam <= s->target_diam && s->cur_total <= s->target_total) s->done = 1;
+    s->temp *= s->cooling;
+    s->step += 1;
   }
-  s->accepted = acc ? 1 : 0;
-  if (s->stop_on_target && s->cur_diam <= s->target_diam && s->cur_total <= s->target_total) s->done = 1;
-  s->temp *= s->cooling;
-  s->step += 1;
+  __syncthreads();
+  for (int i = k; i < s_n; i += blockDim.x)
+    if (!apply_move(s, s->adj, s->edges, s_moves[i])) atomicExch(&s->move_error, 1);
+}
+
+__global__ void decide_kernel(State* __restrict__ s, const Swap* __restrict__ sw, const int* __restrict__ sel,
+                              const BatchOut* __restrict__ out, int K, const Swap* __restrict__ comp,
+                              const BatchOut* __restrict__ comp_out, float* __restrict__ labels,
+                              const Swap* __restrict__ pred, int C) {
+  if (s->done) return;
+  decide_step(s, sw, sel, out, K, comp, comp_out, labels, pred, C);
+}
+
+// The plain step (one candidate, no composites) after its evaluation, in one
+// block: the decision, the best graph's copy and the next step's proposal.  The
+// evaluation patches the proposal into the graph it stages (slice_batch_kernel),
+// so a step is two launches: 23 us at N = 1024, d = 8 in six, 18 us in two.
+// Its one block copies the best edges, so it serves graphs of up to
+// kPlainLines lines.
+constexpr int kPlainLines = 16384;
+__global__ void __launch_bounds__(512) plain_step_kernel(State* __restrict__ s, Swap* __restrict__ sw,
+                                                         const BatchOut* __restrict__ out) {
+  if (s->done) return;   // read by every thread before thread 0 can set it (the barriers of decide_step)
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s->prev_total = s->cur_total;
+    s->best_k = 0;
+    s->n_comp = 0;
+  }
+  __syncthreads();
+  decide_step(s, sw, nullptr, out, 1, nullptr, nullptr, nullptr, nullptr, 0);
+  __syncthreads();
+  if (s->best_step == s->step - 1) {
+    const int n = 2 * s->lines;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) s->best_edges[i] = s->edges[i];
+  }
+  if (threadIdx.x < 32 && !s->done) gen_one(s, sw);
 }
 
 // Copies the current edges to the best edges when this step set a new best.
@@ -541,34 +640,6 @@ __global__ void best_copy_kernel(const State* __restrict__ s) {
 // ---- learned mode: features and selection ---------------------------------------------
 constexpr int kMaxFeatDegree = 32;
 
-// Exact distance d(x, y) read from the base: the first level k whose row x
-// (in the window holding source y) has y's bit, i.e. y in S_k[x].  Window
-// completion bounds the search; a stalled window gives level_cap + 1.
-__device__ int base_distance(const uint4* __restrict__ levels, const int* __restrict__ win_levels, int cap, int N,
-                             int x, int y) {
-  if (x == y) return 0;
-  const int w = y >> 7, b = y & 127;
-  const int L = win_levels[w];
-  const int top = L > 0 ? L : cap;
-  for (int k = 1; k <= top; ++k) {
-    const uint4 r = __ldg(ggb::sub_row(levels, cap, N, w, k, x));
-    const unsigned wd = b < 64 ? (b < 32 ? r.x : r.y) : (b < 96 ? r.z : r.w);
-    if ((wd >> (b & 31)) & 1u) return k;
-  }
-  return cap + 1;
-}
-
-__device__ int common_neighbours(const int* __restrict__ A, int d, int x, int y) {
-  const int* rx = A + (long long)x * d;
-  const int* ry = A + (long long)y * d;
-  int c = 0;
-  for (int i = 0; i < d; ++i) {
-    const int u = rx[i];
-    for (int j = 0; j < d; ++j) c += (ry[j] == u);
-  }
-  return c;
-}
-
 // 32 features per candidate, from the current graph's profile (stats) and
 // adjacency: per endpoint (6 each) eccentricity / 8, mean distance / 8 and
 // log-scaled counts of vertices at distance 2..5; the exact distances (read
@@ -576,129 +647,159 @@ __device__ int common_neighbours(const int* __restrict__ A, int d, int x, int y)
 // cross pairs, / 8;
 // the common-neighbour counts of the pairs it separates; and the
 // transmission gaps of the joined pairs.
-__global__ void features_kernel(const State* __restrict__ s, const Swap* __restrict__ sw, int G,
-                                const unsigned* __restrict__ stats, const uint4* __restrict__ levels,
-                                const int* __restrict__ win_levels, int cap, bf16* __restrict__ X) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+//
+// One warp per candidate: a lane per level of an endpoint's statistics, per
+// (pair, level) of the distances -- d(x, y) is the first level k whose row x
+// holds y's bit; the completion of y's window bounds the search, and a window
+// that stalled gives level_cap + 1 -- and per neighbour.  4096 candidates: 42 us
+// with a thread each (its loads one after the other), 10 us this way.
+__global__ void __launch_bounds__(256) features_kernel(const State* __restrict__ s, const Swap* __restrict__ sw, int G,
+                                                       const unsigned* __restrict__ stats,
+                                                       const uint4* __restrict__ levels,
+                                                       const int* __restrict__ win_levels, int cap,
+                                                       bf16* __restrict__ X) {
+  const int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (k >= G) return;
-  float f[mlp::kFeatures];
-#pragma unroll
-  for (int i = 0; i < mlp::kFeatures; ++i) f[i] = 0.f;
+  const int lane = threadIdx.x & 31;
+  const unsigned all = 0xffffffffu;
+  float f = 0.f;                       // lane i: feature i
   const Swap w = sw[k];
-  if (!s->done && w.valid) {
+  if (!s->done && w.valid) {           // warp-uniform
     const int N = s->N, d = s->d;
     const float inv_logn = 1.f / logf(1.f + (float)N);
+    unsigned st[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) st[e] = stats[(long long)w.x[e] * kStatLevels + lane];
+    // rows of the two separated pairs: lane j holds neighbour j
+    int nb[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) nb[e] = lane < d ? s->adj[(long long)w.x[e] * d + lane] : -1;
+    // distances: pair p of lanes 8p .. 8p + 7, eight levels at a time
+    const int pr = lane >> 3;
+    const int x = pr == 0 || pr == 2 ? w.x[0] : w.x[1], y = pr == 0 || pr == 3 ? w.x[2] : w.x[3];
+    const int L = win_levels[y >> 7], top = L > 0 ? L : cap;
+    int dist = x == y ? 0 : -1;
+    for (int k0 = 1; __any_sync(all, dist < 0); k0 += 8) {
+      const int lv = k0 + (lane & 7);
+      bool hit = false;
+      if (dist < 0 && lv <= top) {
+        const uint4 r = __ldg(ggb::sub_row(levels, cap, N, y >> 7, lv, x));
+        const int b = y & 127;
+        const unsigned wd = b < 64 ? (b < 32 ? r.x : r.y) : (b < 96 ? r.z : r.w);
+        hit = (wd >> (b & 31)) & 1u;
+      }
+      const unsigned m = (__ballot_sync(all, hit) >> (8 * pr)) & 0xffu;
+      if (dist < 0) dist = m ? k0 + __ffs(m) - 1 : k0 + 8 > top ? cap + 1 : -1;
+    }
     float T[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const unsigned* st = stats + (long long)w.x[e] * kStatLevels;
-      int ecc = kStatLevels - 1;
-      double tr = 0.0;
-      for (int q = 0; q < kStatLevels; ++q) {
-        tr += st[q];
-        if (st[q] == 0u && q < ecc) ecc = q;
-      }
-      T[e] = (float)tr;
-      f[6 * e + 0] = (float)ecc * 0.125f;
-      f[6 * e + 1] = (float)(tr / (double)(N - 1)) * 0.125f;
+      // the sum of 32 counts below 2^32: exact in 64 bits, as in a double
+      unsigned long long tr = st[e];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) tr += __shfl_xor_sync(all, tr, o);
+      const unsigned z = __ballot_sync(all, st[e] == 0u);
+      const int ecc = z ? __ffs(z) - 1 : kStatLevels - 1;
+      T[e] = (float)(double)tr;
+      if (lane == 6 * e) f = (float)ecc * 0.125f;
+      if (lane == 6 * e + 1) f = (float)((double)tr / (double)(N - 1)) * 0.125f;
+      const unsigned up = __shfl_up_sync(all, st[e], 1);
+      const float lg = logf(1.f + (float)(up - st[e])) * inv_logn;   // lane q: vertices at distance q
 #pragma unroll
       for (int q = 2; q <= 5; ++q) {
-        const float nq = (float)(st[q - 1] - st[q]);
-        f[6 * e + q] = logf(1.f + nq) * inv_logn;
+        const float v = __shfl_sync(all, lg, q);
+        if (lane == 6 * e + q) f = v;
       }
     }
-    const int* A = s->adj;
-    f[24] = base_distance(levels, win_levels, cap, N, w.x[0], w.x[2]) * 0.125f;
-    f[25] = base_distance(levels, win_levels, cap, N, w.x[1], w.x[3]) * 0.125f;
-    f[26] = base_distance(levels, win_levels, cap, N, w.x[0], w.x[3]) * 0.125f;
-    f[27] = base_distance(levels, win_levels, cap, N, w.x[1], w.x[2]) * 0.125f;
-    f[28] = (float)common_neighbours(A, d, w.x[0], w.x[1]) / (float)d;
-    f[29] = (float)common_neighbours(A, d, w.x[2], w.x[3]) / (float)d;
-    f[30] = fabsf(T[0] - T[2]) / (float)(N - 1);
-    f[31] = fabsf(T[1] - T[3]) / (float)(N - 1);
-  }
-  bf16* row = X + (long long)k * mlp::kFeatures;
 #pragma unroll
-  for (int i = 0; i < mlp::kFeatures; ++i) row[i] = __float2bfloat16_rn(f[i]);
+    for (int p = 0; p < 4; ++p) {
+      const int v = __shfl_sync(all, dist, 8 * p);
+      if (lane == 24 + p) f = v * 0.125f;
+    }
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      int c = 0;
+      for (int j = 0; j < d; ++j) c += nb[2 * p] == __shfl_sync(all, nb[2 * p + 1], j);
+      c = __reduce_add_sync(all, lane < d ? c : 0);
+      if (lane == 28 + p) f = (float)c / (float)d;
+    }
+    if (lane == 30) f = fabsf(T[0] - T[2]) / (float)(N - 1);
+    if (lane == 31) f = fabsf(T[1] - T[3]) / (float)(N - 1);
+  }
+  X[(long long)k * mlp::kFeatures + lane] = __float2bfloat16_rn(f);
 }
 
 // Keeps the K - n_rand candidates with the smallest predicted change
 // (invalid ones last) and n_rand more drawn from the rest, and writes the
-// whole ranking (rank, rank_key) for the predicted composites.  One block of
-// 1024 threads, bitonic sort of G <= kMaxProposals (key, index) pairs.
+// whole ranking (rank, rank_key) for the predicted composites.  Ties go by index.
+// The order is that of the G proposals filled up to a power of two P with
+// entries of index 0 and the invalid proposals' key.
+// An entry's rank is the number of entries before it: kSelRows entries a block,
+// kSelParts threads each over a part of the keys in shared memory.  4096
+// proposals: 60 us as a bitonic sort in one block (78 barriers), 15 us this way.
 constexpr int kMaxProposals = 4096;
-__global__ void __launch_bounds__(1024) select_kernel(const State* __restrict__ s, const Swap* __restrict__ sw,
-                                                      const float* __restrict__ y, int G, int K, int n_rand,
-                                                      int* __restrict__ sel, int* __restrict__ rank,
-                                                      float* __restrict__ rank_key) {
-  __shared__ float s_key[kMaxProposals];
-  __shared__ int s_idx[kMaxProposals];
+constexpr int kSelRows = 32, kSelParts = 16;
+int select_size(int G) {
+  int P = kSelRows;
+  while (P < G) P <<= 1;
+  return P;
+}
+__global__ void __launch_bounds__(kSelRows * kSelParts) select_kernel(const State* __restrict__ s,
+                                                                     const Swap* __restrict__ sw,
+                                                                     const float* __restrict__ y, int G, int K,
+                                                                     int n_rand, int* __restrict__ sel,
+                                                                     int* __restrict__ rank,
+                                                                     float* __restrict__ rank_key) {
+  __shared__ unsigned long long s_key[kMaxProposals];   // ordered key, the index it stands for, its own
+  __shared__ int s_target[kComposeThreads];             // ranks of the random picks
   if (s->done) return;
   int P = 1;
   while (P < G) P <<= 1;
-  for (int i = threadIdx.x; i < P; i += blockDim.x) {
-    const bool ok = i < G && sw[i].valid;
-    s_key[i] = ok ? y[i] : FLT_MAX;
-    s_idx[i] = i < G ? i : 0;
+  const int tid = threadIdx.x, top = K - n_rand;
+  auto value = [&](int i) { return i < G && sw[i].valid ? y[i] : FLT_MAX; };
+  for (int i = tid; i < P; i += blockDim.x) {
+    const float v = value(i);
+    const unsigned b = __float_as_uint(v == 0.f ? 0.f : v);   // -0 and 0 are equal
+    const unsigned o = (b & 0x80000000u) ? ~b : b | 0x80000000u;
+    s_key[i] = ((unsigned long long)o << 32) | ((unsigned)(i < G ? i : 0) << 16) | (unsigned)i;
+  }
+  for (int q = tid; q < n_rand; q += blockDim.x) {
+    const unsigned long long h =
+        draw(s->seed ^ 0x243f6a8885a308d3ULL, (unsigned long long)s->step, 0x5e1ecULL, top + q);
+    s_target[q] = top + below(h, G - top);
   }
   __syncthreads();
-  for (int size = 2; size <= P; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = threadIdx.x; i < P; i += blockDim.x) {
-        const int j = i ^ stride;
-        if (j > i) {
-          const bool up = (i & size) == 0;
-          const float ki = s_key[i], kj = s_key[j];
-          const int ii = s_idx[i], ij = s_idx[j];
-          const bool gt = ki > kj || (ki == kj && ii > ij);
-          if (gt == up) {
-            s_key[i] = kj; s_key[j] = ki;
-            s_idx[i] = ij; s_idx[j] = ii;
-          }
-        }
-      }
-      __syncthreads();
-    }
+  const int i = blockIdx.x * kSelRows + tid / kSelParts, part = tid % kSelParts;
+  const unsigned long long me = i < P ? s_key[i] : 0ULL;
+  int before = 0;
+#pragma unroll 8
+  for (int j = part; j < P; j += kSelParts) before += s_key[j] < me;
+#pragma unroll
+  for (int o = kSelParts / 2; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  if (i >= P || before >= G) return;
+  const int c = i < G ? i : 0;
+  if (part == 0) {
+    rank[before] = c;
+    rank_key[before] = value(i);
+    if (before < top) sel[before] = c;
   }
-  for (int q = threadIdx.x; q < G; q += blockDim.x) {
-    rank[q] = s_idx[q];
-    rank_key[q] = s_key[q];
-  }
-  const int top = K - n_rand;
-  for (int q = threadIdx.x; q < K; q += blockDim.x) {
-    if (q < top) {
-      sel[q] = s_idx[q];
-    } else {
-      const unsigned long long h = draw(s->seed ^ 0x243f6a8885a308d3ULL, (unsigned long long)s->step, 0x5e1ecULL, q);
-      sel[q] = s_idx[top + below(h, G - top)];
-    }
-  }
+  for (int q = part; q < n_rand; q += kSelParts)
+    if (s_target[q] == before) sel[top + q] = c;
 }
 
 // The predicted list: walking the ranking best first, every valid proposal
 // predicted to lower the distance total (key < 0) whose endpoints are not
-// yet used, up to pred_max swaps.  One thread.
+// yet used, up to pred_max swaps.  One warp: 25 us for 4096 proposals at N = 16384 (78 us with one thread).
 __global__ void pred_list_kernel(State* __restrict__ s, const Swap* __restrict__ sw, const int* __restrict__ rank,
                                  const float* __restrict__ rank_key, int G, int pred_max, Swap* __restrict__ pred,
                                  unsigned* __restrict__ vmark) {
-  if (s->done || threadIdx.x != 0) return;
-  int m = 0;
-  for (int r = 0; r < G && m < pred_max; ++r) {
-    if (!(rank_key[r] < 0.f)) break;   // sorted: no further predicted gain
-    const Swap w = sw[rank[r]];
-    if (!w.valid) continue;
-    int cl[4];
-    const int nc = move_classes(s, w, cl);
-    if (!classes_free(vmark, cl, nc)) continue;
-    classes_set(vmark, cl, nc, true);
-    pred[m++] = w;
-  }
-  for (int i = 0; i < m; ++i) {
-    int cl[4];
-    const int nc = move_classes(s, pred[i], cl);
-    classes_set(vmark, cl, nc, false);
-  }
-  s->n_pred = m;
+  if (s->done) return;
+  const int m = greedy_disjoint(s, vmark, G, pred_max, pred, [&](int r, Swap& w) -> int {
+    if (!(rank_key[r] < 0.f)) return 0;   // sorted: no further predicted gain
+    w = sw[rank[r]];
+    return w.valid ? 2 : 1;
+  });
+  if (threadIdx.x == 0) s->n_pred = m;
 }
 
 // The composite batch: slot 0 the exact composite, slot 1 + c predicted
@@ -740,6 +841,7 @@ struct ggb_sa {
   int C = 0, pred_max = 0;        // predicted composites (learned mode) and their largest size
   bool learned = false;
   bool delta = false;             // candidates evaluated against the base, not in full
+  bool plain = false;             // the captured step is the two-launch plain step
   bool has_base = false;          // the base is kept (delta evaluation, the filter's features)
   bool broken = false;            // a restore failed while re-sizing the base: only destroy is allowed
   State h{};                      // host mirror of the device state
@@ -976,16 +1078,24 @@ int enqueue_step(ggb_sa* a, cudaStream_t st) {
   using namespace ggb::sa;
   State* s = a->d_state;
   const int G = a->learned ? a->G : a->K;
+  if (a->plain) {   // the proposal is there: drawn by the step before, or by ggb_sa_run
+    int rc = ggb::batch_enqueue(a->cand, st);
+    if (rc) return rc;
+    plain_step_kernel<<<1, 512, 0, st>>>(s, a->d_swaps, a->cand->d_out);
+    ggb::core_add_launches(2);
+    SCUDA(cudaGetLastError());
+    return GGB_OK;
+  }
   gen_kernel<<<(G + 127) / 128, 128, 0, st>>>(s, a->d_swaps, G);
   int launches = 1;
   const int* sel = nullptr;
   if (a->learned) {
-    features_kernel<<<(G + 127) / 128, 128, 0, st>>>(s, a->d_swaps, G, a->d_stats, a->d_levels, a->d_winlev,
-                                                     a->level_cap, a->d_X);
+    features_kernel<<<(G + 7) / 8, 256, 0, st>>>(s, a->d_swaps, G, a->d_stats, a->d_levels, a->d_winlev,
+                                                 a->level_cap, a->d_X);
     int rc = ggb::mlp_forward(a->mlp, a->d_X, G, a->d_scores, st);
     if (rc) return rc;
-    select_kernel<<<1, 1024, 0, st>>>(s, a->d_swaps, a->d_scores, G, a->K, a->n_rand, a->d_sel, a->d_rank,
-                                      a->d_rank_key);
+    select_kernel<<<select_size(G) / kSelRows, kSelRows * kSelParts, 0, st>>>(
+        s, a->d_swaps, a->d_scores, G, a->K, a->n_rand, a->d_sel, a->d_rank, a->d_rank_key);
     sel = a->d_sel;
     launches += 2;
   }
@@ -996,17 +1106,23 @@ int enqueue_step(ggb_sa* a, cudaStream_t st) {
     if (rc) return rc;
     singles = a->d_dout;
   } else {
-    const long long stride = a->cand->off.size() > 1 ? a->cand->off[1] - a->cand->off[0] : 0;
-    const int bx = std::max(1, std::min(a->sms * 4 / std::max(a->K, 1), (int)(((long long)a->N * a->d + 255) / 256)));
-    materialize_kernel<<<dim3(bx, a->K), 256, 0, st>>>(s, a->d_swaps, sel, a->cand->d_adj, stride);
-    if (a->groups > 1) {
-      patch_orbit_kernel<<<a->K, 32, 0, st>>>(s, a->d_swaps, sel, a->cand->d_adj, stride);
+    // candidates on slices are patched into the graph as it is staged
+    const bool patched = a->groups == 1 && !sel && a->cand->all_slices();
+    a->cand->patch_base = patched ? a->d_adj : nullptr;
+    a->cand->patch = patched ? a->d_swaps : nullptr;
+    if (!patched) {
+      const long long stride = a->cand->off.size() > 1 ? a->cand->off[1] - a->cand->off[0] : 0;
+      const int bx = std::max(1, std::min(a->sms * 4 / std::max(a->K, 1), (int)(((long long)a->N * a->d + 255) / 256)));
+      materialize_kernel<<<dim3(bx, a->K), 256, 0, st>>>(s, a->d_swaps, sel, a->cand->d_adj, stride);
       launches += 1;
+      if (a->groups > 1) {
+        patch_orbit_kernel<<<a->K, 32, 0, st>>>(s, a->d_swaps, sel, a->cand->d_adj, stride);
+        launches += 1;
+      }
     }
     rc = ggb::batch_enqueue(a->cand, st);
     if (rc) return rc;
     singles = a->cand->d_out;
-    launches += 1;
   }
   compose_kernel<<<1, kComposeThreads, 0, st>>>(s, a->d_swaps, sel, singles, a->K, a->d_comp, a->compose_max,
                                                 a->d_vmark);
@@ -1052,6 +1168,12 @@ int enqueue_step(ggb_sa* a, cudaStream_t st) {
 
 int capture_step(ggb_sa* a) {
   if (a->exec) return GGB_OK;
+  a->plain = a->K == 1 && a->groups == 1 && !a->comp && !a->has_base && !a->learned && a->cand->all_slices() &&
+             a->lines <= ggb::sa::kPlainLines;
+  if (a->plain) {
+    a->cand->patch_base = a->d_adj;
+    a->cand->patch = a->d_swaps;
+  }
   SCUDA(cudaStreamBeginCapture(a->st, cudaStreamCaptureModeThreadLocal));
   int rc = enqueue_step(a, a->st);
   cudaGraph_t gph = nullptr;
@@ -1639,6 +1761,7 @@ int ggb_sa_autotune(ggb_sa* a, int iters, int* window_bits, int* team_ctas, doub
   SCUDA(cudaSetDevice(a->device));
   drop_graph(a);
   ggb_batch* b = a->cand ? a->cand : a->comp;
+  if (a->cand) a->cand->patch_base = nullptr;   // the batch is timed on its own adjacencies
   if (!b) {
     if (window_bits) *window_bits = 0;
     if (team_ctas) *team_ctas = 0;
@@ -1654,6 +1777,11 @@ int ggb_sa_run(ggb_sa* a, long long steps, ggb_sa_stats* stats) {
   SCUDA(cudaSetDevice(a->device));
   int rc = capture_step(a);
   if (rc) return rc;
+  if (a->plain) {   // the first step's proposal; every step draws the next one's
+    ggb::sa::gen_kernel<<<1, 32, 0, a->st>>>(a->d_state, a->d_swaps, 1);
+    ggb::core_add_launches(1);
+    SCUDA(cudaGetLastError());
+  }
   for (long long i = 0; i < steps; ++i) SCUDA(cudaGraphLaunch(a->exec, a->st));
   SCUDA(cudaStreamSynchronize(a->st));
   rc = check_sticky(a);
