@@ -15,7 +15,8 @@ struct ggb_batch {
   size_t l2 = 0;
   int n = 0;
   std::vector<int> N, bn, grp, d;
-  std::vector<long long> off;        // ints; every graph starts on a 16-byte boundary
+  std::vector<int> by_size;          // graphs in order of N: the order of their adjacencies
+  std::vector<long long> off;        // ints; a multiple of 8 (16-byte boundaries in d_adj16 as well)
   long long adj_ints = 0;
   int* d_adj = nullptr;
   int* h_adj = nullptr;              // pinned staging for ggb_batch_eval
@@ -68,7 +69,10 @@ struct ggb_batch {
   cudaStream_t stream = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  cudaEvent_t ev[2] = {nullptr, nullptr};
+  cudaStream_t copies = nullptr;     // uploads beside running kernels (eval_parts)
+  cudaEvent_t arrived = nullptr;
+  cudaEvent_t ev[6] = {};            // around each of the last evaluation's `timed` launches
+  int timed = 0;
   bool pending = false;
   // Graph i is patch_base with patch[i] applied instead of its own adjacency
   // (device; only while every graph is on slices, see all_slices).
@@ -81,9 +85,12 @@ struct ggb_batch {
 
 namespace ggb {
 
+// The parts of an evaluation, in the order batch_enqueue() takes them.
+enum { kPartClear = 1, kPartLevels = 2, kPartWindows = 4, kPartSlices = 8, kPartAll = 15 };
+
 // Enqueues one evaluation of the batch's device adjacency on `st` (zeroing
-// of the control blocks and results, then the cooperative kernel); usable
-// inside a stream capture.
-int batch_enqueue(ggb_batch* b, cudaStream_t st);
+// of the control blocks and results, then the kernels), or some parts of it;
+// usable inside a stream capture.
+int batch_enqueue(ggb_batch* b, cudaStream_t st, int parts = kPartAll);
 
 }  // namespace ggb
