@@ -147,16 +147,26 @@ double make_plan(ggb_batch* b, const std::vector<int>& ids, int R, int T, bool k
     pq.push(l);
   }
   // Working set of the teams running at once: each team's adjacency and two
-  // matrices.  Past the L2 size the gathers spill to HBM, at a mild price (51
-  // graphs of 8192 to 16384 vertices, R = 32: 3.8 ms on 6 teams of 24 CTAs,
-  // 100 MB, 4.4 ms on 18 of 8, 315 MB).
+  // matrices.  Past 60 % of L2 the gathers begin to spill to HBM: a steep price
+  // up to about 8500 vertices (22 graphs of 81 to 8357, d = 16: 464 us with it, 525
+  // without), a mild one above (51 graphs of 8192 to 16384 vertices, R = 32: 3.8 ms on 6
+  // teams of 24 CTAs, 100 MB, 4.4 ms on 18 of 8, 315 MB).
   double ws = 0.0;
+  int largest = 0;
   for (int t = 0; t < n_teams; ++t) {
     long long mx = 0;
-    for (int i : lists[t]) mx = std::max<long long>(mx, (long long)b->N[i] * (b->d[i] * 4 + 32 * R));
+    for (int i : lists[t]) {
+      mx = std::max<long long>(mx, (long long)b->N[i] * (b->d[i] * 4 + 32 * R));
+      largest = std::max(largest, b->N[i]);
+    }
     ws += (double)mx;
   }
-  if (ws > (double)b->l2) makespan *= 1.0 + 0.12 * (ws / (double)b->l2 - 1.0);
+  const double l2 = (double)b->l2;
+  if (largest <= 8500) {
+    if (ws > 0.6 * l2) makespan *= 1.0 + 1.5 * std::min(1.0, (ws - 0.6 * l2) / (0.6 * l2));
+  } else if (ws > l2) {
+    makespan *= 1.0 + 0.12 * (ws / l2 - 1.0);
+  }
   if (!keep) return makespan;
   b->R = R;
   b->T = T;
@@ -383,6 +393,15 @@ int plan_split(ggb_batch* b) {
     if ((long long)N * (d + 1) <= most && N <= ggb::kSliceMaxN && smem <= kSliceSmemMax) small.push_back(i);
     else if (b->grp[i] == 1 && d >= 4 && d <= 32 && N > from && N <= 22000) mid.push_back(i);
     else rest.push_back(i);
+  }
+  // The kernels follow one another and each has its tail.  With graphs for the
+  // level-by-level teams the split pays (1.0 to 2.1 times); with small
+  // graphs beside window teams only it does not always (29 graphs of 109 to 5162
+  // vertices, d = 15: 625 us, 529 on teams alone; 89 of 86 to 4844, d = 14: 1050,
+  // 925; 16 of 540 to 4897, d = 15: 395, 556): those stay on teams.
+  if (mid.empty() && !rest.empty()) {
+    rest = all_graphs(b);
+    small.clear();
   }
   plan_slices(b, small);
   plan_levels(b, mid);
