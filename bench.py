@@ -6,13 +6,14 @@ N = 65536 vertices (int32 adjacency [65536][16], 4 MiB), all 65536 sources,
 g = 1.  A step is one complete exact evaluation (diameter, integer distance
 total, ASPL) of that graph.
 
-* ``value``  -- evals/s with the adjacency already in HBM: the persistent
-  kernel timed with CUDA events on its launching stream, the L2 flushed
+* ``value``  -- evals/s with the adjacency already in HBM: all kernels of an
+  evaluation timed with CUDA events on their launching stream, the L2 flushed
   (a 512 MiB write) before every step, outside the events.
 * ``e2e``    -- the same metric through the public C ABI with host buffers
   (ggb_eval_general: pinned staging, H2D of the adjacency, kernel, D2H of the
   result block, synchronise), wall-clock per call.
-* ``roofline`` -- the dominant kernel (the persistent sweep kernel): its
+* ``roofline`` -- the dominant kernel (the half sweeps of a symmetric graph at
+  the automatic width, the persistent sweep kernel at forced ones): its
   algorithmic bytes (per dense sweep: N*d*4 adjacency + N*d*W/8 gathered rows
   + N*W/8 own row read + N*W/8 write) over its own event-timed duration
   (events recorded by the library on the launching stream), against the
@@ -224,8 +225,8 @@ def roofline(kernel: str, alg: float, ms: float, l2_roof, hbm_peak: float, hbm_k
     if lts_pct is not None:
         out["lts_throughput_pct"] = lts_pct
     out["note"] = ("achieved counts every gather of every dense sweep (the reference algorithm's bytes), "
-                   "including the parts the fullness checks and full-row stamps skip, so it can read a little "
-                   "above the ceiling; frac_of_l2_stream is the physical L2 rate against it; traffic = DRAM "
+                   "including the rows that half sweeps take from transposes and the parts that fullness "
+                   "checks and full-row stamps skip, so it can read above the ceiling; frac_of_l2_stream is the physical L2 rate against it; traffic = DRAM "
                    "bytes per launch from the committed ncu capture under profiles/")
     return out
 
@@ -546,14 +547,15 @@ def main() -> int:
     e2e_value = world * args.steps / e2e_max
 
     peak, peak_kind = _peaks()
-    # dominant kernel: the persistent kernel (dense sweeps); the ball pre-pass is reported beside it
+    # dominant kernel: the dense sweeps; the ball pre-pass is reported beside it
     pers_ms = statistics.mean(kt_pers) if kt_pers else mean_ms
     ball_ms = statistics.mean(kt_ball) if kt_ball else 0.0
     alg = sweep_bytes(n, d, first.dense_levels, first.window_bits)
     achieved = alg / (pers_ms / 1e3) / 1e9
     l2_roof = l2_gather_roof(lib, n, d, first.window_bits)
     prof = _profile(args.workload)
-    kp = prof.get("apsp_persistent_kernel", {})
+    main = "apsp_sym_kernel" if "apsp_sym_kernel" in prof and not args.window_bits else "apsp_persistent_kernel"
+    kp = prof.get(main, {})
     traffic = kp.get("dram_bytes_per_launch")
     lts = kp.get("lts_bytes_per_launch")
 
@@ -565,13 +567,14 @@ def main() -> int:
             "run": {"sources": bn, "window_bits": first.window_bits, "windows": first.windows,
                     "levels": first.levels, "dense_levels": first.dense_levels,
                     "diameter": first.diameter, "total": first.total, "aspl": first.aspl},
-            "roofline": roofline(f"apsp_persistent_kernel<{first.window_bits // 128}>", alg, pers_ms, l2_roof,
+            "roofline": roofline(f"{main}<{first.window_bits // 128}>", alg, pers_ms, l2_roof,
                                  peak, peak_kind, traffic, lts, kp.get("lts_throughput_pct"),
                                  l2_stream_roof(lib)),
             "ball_prepass": {"ms_per_launch": ball_ms,
                              "algorithmic_bytes_per_launch": ball_bytes(n, d, first.windows, first.window_bits)
                              if ball_ms else 0,
-                             "traffic": prof.get("ball_kernel", {}).get("dram_bytes_per_launch")},
+                             "traffic": prof.get("sym_ball_kernel" if main == "apsp_sym_kernel" else "ball_kernel",
+                                                 {}).get("dram_bytes_per_launch")},
             "survey_formula_bytes_per_eval": survey_formula_bytes(n, d, first.levels, first.window_bits),
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d_per_step),
                     "d2h_bytes_per_step": 96, "input_bytes_per_step": n * d * 4,
@@ -713,7 +716,10 @@ def batch_bench(peak: float, peak_kind: str, lib) -> dict:
     alg = sum(sweep_bytes(x.nodes, 12, r.dense_levels, r.window_bits) for x, r in zip(w, res))
     l2 = l2_gather_roof(lib, 16384, 12, bits)
     b.close()
-    roof = roofline(f"apsp_batch_kernel<{bits // 128}>", alg, kms, l2, peak, peak_kind, None, None,
+    mixed = len({r.window_bits for r in res}) > 1   # the automatic plan: three kernels
+    kernel = ("slice_batch_kernel + apsp_batch_levels_kernel + apsp_batch_kernel" if mixed
+              else f"apsp_batch_kernel<{bits // 128}>")
+    roof = roofline(kernel, alg, kms, l2, peak, peak_kind, None, None,
                     l2_stream=l2_stream_roof(lib))
     roof["l2_gather_probe_case"] = "N=16384, d=12: the largest graphs of the batch"
     return {"workload": "4096-vertex base + 256 single-swap candidates, d=12, N log-uniform 512..16384",

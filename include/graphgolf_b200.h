@@ -51,10 +51,11 @@ typedef struct ggb_result {
                            `sum += nodes*(nodes-1)`; 0 if disconnected        */
   long long levels;     /* BFS levels executed, summed over source windows   */
   int windows;          /* source windows run                                 */
-  int window_bits;      /* sources per window (64 or a multiple of 128)       */
+  int window_bits;      /* sources per window (32, 64 or a multiple of 128)   */
   long long dense_levels; /* of `levels`, those run as dense OR-gather sweeps
-                           (the first two levels of a window are seeded from
-                           the two-hop adjacency instead)                     */
+                           (the first levels of a window may be seeded from
+                           the two-hop adjacency, the last ones of a symmetric
+                           graph taken pair by pair)                          */
 } ggb_result;
 
 /* Partial result of a rank that ran a strided share of the source windows
@@ -124,7 +125,7 @@ int ggb_trace_enable(int capacity);
 int ggb_trace_read(long long *out, int max_pairs);
 
 /* Per-kernel timing: with enable != 0, CUDA events are recorded on the
- * launching stream around the ball pre-pass and the persistent kernel of
+ * launching stream around the ball pre-pass and the sweep kernel of
  * every following evaluation; ggb_kernel_times returns the last one's
  * milliseconds (ball 0 when it did not run).  No counterpart in the
  * reference; bench.py's roofline uses it. */
@@ -198,7 +199,7 @@ int ggb_launch_general_device(int nodes, int based_nodes, int groups, int degree
 int ggb_collect(void *stream, ggb_result *out);
 
 /* Number of this library's kernels enqueued since load: every kernel of an
- * evaluation (ball pre-pass, persistent kernel, the grid relabel kernels, the
+ * evaluation (ball pre-pass, sweep kernels, the grid relabel kernels, the
  * widening of 16-bit ids after an upload) counts once per launch. */
 long long ggb_kernel_launches(void);
 
@@ -257,11 +258,13 @@ int ggb_finish_grid(int nodes, const ggb_partial *reduced, ggb_result *out);
 /* ---- batches: many graphs, of uneven sizes, in one launch --------------- */
 
 /* A batch is a fixed list of general graphs (ac = 0) whose adjacency arrays
- * live packed in one device buffer; one cooperative launch, captured once in a
- * CUDA graph and replayed, evaluates them all.  Its CTAs form teams of
- * team_ctas CTAs; the graphs are dealt to the teams longest-first; every team
- * runs its graphs' source windows of window_bits sources with a barrier of its
- * own.  Each graph's result is the one ggb_eval_general gives it
+ * live packed in one device buffer.  The launches, captured once in a CUDA
+ * graph and replayed, evaluate them all.  The automatic plan takes small graphs
+ * in shared memory, mid-size ones level by level on teams of CTAs, and the rest
+ * as source windows on teams.  A fixed plan takes every graph the last way, in
+ * one cooperative launch: its CTAs form teams of team_ctas CTAs, the graphs are
+ * dealt to the teams longest-first, and every team runs its graphs' source
+ * windows of window_bits sources with a barrier of its own.  Each graph's result is the one ggb_eval_general gives it
  * (general/evaluation.c:153-263 per graph, :249-262 for the convention).  No
  * counterpart in the reference, whose evaluation() takes one graph.
  * A batch belongs to the device current at ggb_batch_create; it is not
@@ -270,18 +273,20 @@ typedef struct ggb_batch ggb_batch;
 
 /* Creates a batch of n_graphs graphs; graph i has nodes[i] vertices,
  * based_nodes[i] * groups[i] == nodes[i], degree[i] neighbours per row.  The
- * initial plan is the cost model's choice. */
+ * initial plan is the automatic one. */
 int ggb_batch_create(int n_graphs, const int *nodes, const int *based_nodes, const int *groups,
                      const int *degree, ggb_batch **out);
 void ggb_batch_destroy(ggb_batch *b);
 
 /* Fixes the plan: window_bits = 128 * 2^k (<= 4096), team_ctas >= 1; a 0
- * leaves that choice to the cost model. */
+ * leaves that choice to the cost model, two 0s are the automatic plan.
+ * ggb_batch_get_plan reports, for the automatic plan, its window teams, or its
+ * level-by-level teams when it has no window teams, or its shared-memory windows. */
 int ggb_batch_set_plan(ggb_batch *b, int window_bits, int team_ctas);
 int ggb_batch_get_plan(const ggb_batch *b, int *window_bits, int *team_ctas, int *teams);
 
-/* Times every feasible (window_bits, team_ctas) pair on the batch's current
- * adjacency (iters timed launches each, after one warm-up) and keeps the
+/* Times the automatic plan and every feasible (window_bits, team_ctas) pair on
+ * the batch's current adjacency (iters timed launches each, after one warm-up) and keeps the
  * fastest; reports it and its time. */
 int ggb_batch_autotune(ggb_batch *b, int iters, int *window_bits, int *team_ctas, double *best_ms);
 
@@ -299,10 +304,12 @@ int ggb_batch_upload(ggb_batch *b, const int *const *adj, void *stream);
 int ggb_batch_launch(ggb_batch *b, void *stream);
 int ggb_batch_collect(ggb_batch *b, void *stream, ggb_result *results);
 
-/* Upload + launch + collect. */
+/* Upload + launch + collect; with the automatic plan each kernel is launched
+ * once its graphs have arrived, beside the upload of the next one's. */
 int ggb_batch_eval(ggb_batch *b, const int *const *adj, ggb_result *results);
 
-/* Device time of the last collected launch (CUDA events around it). */
+/* Device time of the last collected evaluation's launches (CUDA events around
+ * them; waits for uploads between them are not counted). */
 int ggb_batch_kernel_ms(const ggb_batch *b, double *ms);
 
 /* ---- the proposal filter's network (learned annealing) ------------------ */
