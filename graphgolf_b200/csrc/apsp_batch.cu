@@ -825,8 +825,7 @@ void model_choice(ggb_batch* b, const std::vector<int>& ids, int* R, int* T) {
   int nsrc_max = 0;
   for (int i : ids) nsrc_max = std::max(nsrc_max, b->bn[i]);
   for (int r = 1; r <= kMaxR; r *= 2) {
-    for (int t : {1, 2, 4, 8, 16, 24, 37, 49, 74, 148}) {
-      if (t > b->occ[log2i(r)] * b->sms) break;
+    for (int t = 1; t <= b->occ[log2i(r)] * b->sms; t *= 2) {
       const double m = make_plan(b, ids, r, t, false);
       if (m < best * 0.999) { best = m; *R = r; *T = t; }
     }

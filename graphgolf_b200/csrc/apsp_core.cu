@@ -710,8 +710,13 @@ int launch_sym(const SymPlan& pl, const int* d_adj, int N, int d, cudaStream_t s
 // Measured (whole call, us, level by level / half-sweep windows / persistent
 // kernel): N = 8500, d = 12 110 / - / 147; 12000, d = 12 135 / 143 / 180;
 // 12000, d = 32 124 / - / 216; 16384, d = 12 180 / 187 / 216; 18000, d = 12
-// 219 / 216; 22000, d = 16 229 / 247; 8192, d = 12 109 / - / 81.
+// 219 / 216; 22000, d = 16 229 / 247; 8192, d = 12 109 / - / 81.  Low degrees
+// have more levels, each with its two barriers, and around 13 000 vertices the
+// persistent kernel's windows fit best (level by level / persistent kernel):
+// d = 4: 10000 216 / 222, 12000 246 / 236, 13400 266 / 243, 15400 278 / 295;
+// d = 6: 12000 182 / 212, 13400 209 / 195, 15400 207 / 211.
 bool levels_served(int N, int d) {
+  if (d <= 6 && N > 12300 && N <= 15000) return false;
   return slices_allowed() && d >= 4 && d <= 32 && N > 8192 && N <= (d >= 16 ? 22000 : 18000);
 }
 
