@@ -135,6 +135,7 @@ __device__ __forceinline__ void levels_sweep(const SymArgs& s, const uint4* __re
                                              const int* __restrict__ adj, int N, int d, int vec4, int C, bool early,
                                              long long warp_id, long long n_warps, unsigned& c_diag, unsigned& c_off) {
   constexpr int U = 8;
+  bool full = false;
   const int lane = threadIdx.x & 31, h = lane >> 4, hl = lane & 15;
   // half-warp tasks: row v of the column group i (16 parts, 4096 bits), v >= 4096 i
   const int groups = (C / 2 + 15) / 16;
@@ -193,7 +194,7 @@ __device__ __forceinline__ void levels_sweep(const SymArgs& s, const uint4* __re
     if (p == dp) c_diag += cc; else c_off += cc;
     if constexpr (LAST) {
       if (cc != (unsigned)nv)
-        for (int k = 0; k < 8; ++k) list_missing(s, word_of(acc, k), nv - 32 * k, v, 256 * p + 32 * k, p == dp, kLevelsList);
+        for (int k = 0; k < 8; ++k) list_missing(s, word_of(acc, k), nv - 32 * k, v, 256 * p + 32 * k, p == dp, full, kLevelsList);
     } else {
       st_cg2(dst + (size_t)v * C + col, acc);
     }

@@ -231,9 +231,14 @@ __device__ __forceinline__ void transpose_tile(const uint4* __restrict__ src, si
 
 // ---- one half sweep -----------------------------------------------------------------
 // Appends the unset bits among the `nv` valid ones of word `x` (bit b is
-// source s0 + b) of row v; in the diagonal block only sources below v.
+// source s0 + b) of row v; in the diagonal block only sources below v.  A
+// thread that has seen the list full (`full`) appends no more: the unreached
+// pairs of a graph whose first window lies close to everything while the others
+// do not can exceed 2^32 (from 92 682 vertices on), but the counter ends below
+// cap + 32 a thread.
 __device__ __forceinline__ void list_missing(const SymArgs& s, unsigned x, int nv, int v, int s0, bool diag,
-                                             unsigned cap = kSymList) {
+                                             bool& full, unsigned cap = kSymList) {
+  if (full) return;
   unsigned m = ~x & (nv >= 32 ? 0xffffffffu : (1u << max(nv, 0)) - 1u);
   if (diag) {
     const int b = v - s0;                       // sources s0 .. v - 1
@@ -241,6 +246,7 @@ __device__ __forceinline__ void list_missing(const SymArgs& s, unsigned x, int n
   }
   if (!m) return;
   unsigned at = atomicAdd(s.list_n, (unsigned)__popc(m));
+  full = at >= cap;
   while (m) {
     const int b = __ffs(m) - 1;
     m &= m - 1;
@@ -270,7 +276,7 @@ template <int R, bool LAST>
 __device__ __forceinline__ void sym_sweep(const SymArgs& s, const SymRows src, uint4* __restrict__ lo,
                                           uint4* __restrict__ hi, const int* __restrict__ adj, int N, int d, int vec4,
                                           int first, int v_next, int l, bool early, long long warp_id,
-                                          long long n_warps, unsigned& c_diag, unsigned& c_off) {
+                                          long long n_warps, unsigned& c_diag, unsigned& c_off, bool& full) {
   constexpr int LP = R / 2 < 32 ? R / 2 : 32;     // lanes a row
   constexpr int PPL = R / (2 * LP);               // 32-byte parts a lane
   constexpr int G = 32 / LP;                      // rows a warp and step
@@ -344,7 +350,7 @@ __device__ __forceinline__ void sym_sweep(const SymArgs& s, const SymRows src, u
         const int b0 = 256 * (hl + p * LP);        // first bit of the part
         const int nv = min(256, l - b0);
         if (nv > 0 && popc4(acc[p][0]) + popc4(acc[p][1]) != (unsigned)nv)
-          for (int k = 0; k < 8; ++k) list_missing(s, word_of(acc[p], k), nv - 32 * k, v, first + b0 + 32 * k, diag);
+          for (int k = 0; k < 8; ++k) list_missing(s, word_of(acc[p], k), nv - 32 * k, v, first + b0 + 32 * k, diag, full);
       }
     } else {
 #pragma unroll
@@ -419,7 +425,7 @@ __device__ __forceinline__ bool grid_wait(ApspCtrl* c, unsigned long long target
 // Lists the unreached pairs of window 0 from its rows at level k*.
 template <int R>
 __device__ __forceinline__ void sym_list_window0(const SymArgs& s, const SymRows rows, int N, int l,
-                                                 long long warp_id, long long n_warps) {
+                                                 long long warp_id, long long n_warps, bool& full) {
   constexpr int LP = R / 2 < 32 ? R / 2 : 32, PPL = R / (2 * LP), G = 32 / LP;
   const int lane = threadIdx.x & 31, h = lane / LP, hl = lane % LP;
   for (long long vb = warp_id * G; vb + h < N; vb += n_warps * G) {
@@ -430,7 +436,7 @@ __device__ __forceinline__ void sym_list_window0(const SymArgs& s, const SymRows
       ld_cg2((v < rows.split ? rows.lo : rows.hi) + (size_t)v * R + 2 * (hl + p * LP), x);
       const int b0 = 256 * (hl + p * LP), nv = min(256, l - b0);
       if (nv > 0 && popc4(x[0]) + popc4(x[1]) != (unsigned)nv)
-        for (int k = 0; k < 8; ++k) list_missing(s, word_of(x, k), nv - 32 * k, v, b0 + 32 * k, v < l);
+        for (int k = 0; k < 8; ++k) list_missing(s, word_of(x, k), nv - 32 * k, v, b0 + 32 * k, v < l, full);
     }
   }
 }
@@ -530,6 +536,7 @@ __global__ void __launch_bounds__(kThreads, 1) apsp_sym_kernel(const ApspArgs a,
   unsigned early = 0u;                                 // levels made from one that is nearly full
   int sweeps = 0;
   unsigned q = 0;                                      // dense writes so far: the buffer in turn
+  bool full = false;                                   // this thread has seen the list full
   if (!fallback) {
     const int l = min(W, N);
     // row v of window k at a stored level lies at level + tri_base(k) + v * R, from (k + 1) * W on
@@ -546,7 +553,7 @@ __global__ void __launch_bounds__(kThreads, 1) apsp_sym_kernel(const ApspArgs a,
       uint4* const hi = L - kSymFirst < s.stored ? s.tri + (size_t)(L - kSymFirst) * s.tri_cells + tri_base(0) : dst;
       unsigned cd = 0, co = 0;
       sym_sweep<R, false>(s, src, dst, hi, a.adj, N, d, a.vec4, 0, l, l, (early >> L) & 1u, warp_id,
-                          n_warps, cd, co);
+                          n_warps, cd, co, full);
       ++sweeps;
       sym_add((unsigned long long)cd + co, s.cnt + kSymCnt0 + L);
       // the weighted count holds rows of the window's own block once, the others twice
@@ -582,13 +589,13 @@ __global__ void __launch_bounds__(kThreads, 1) apsp_sym_kernel(const ApspArgs a,
       nbuf = last - kSymFirst >= 3 ? 4 : 3;
       auto finish = [&](int i, const SymRows from) {
         if (i == 0) {
-          sym_list_window0<R>(s, from, N, l, warp_id, n_warps);
+          sym_list_window0<R>(s, from, N, l, warp_id, n_warps, full);
           return;
         }
         const int first = i * W, li = min(W, N - first);
         unsigned cd = 0, co = 0;
         sym_sweep<R, true>(s, from, nullptr, nullptr, a.adj, N, d, a.vec4, first, first + li, li, (early >> last) & 1u,
-                           warp_id, n_warps, cd, co);
+                           warp_id, n_warps, cd, co, full);
         sym_add((unsigned long long)cd + 2ull * co, s_acc + last);
       };
       SymRows done = src;                              // rows of window i - 1 one level below k* (window 0: at k*)
@@ -606,7 +613,7 @@ __global__ void __launch_bounds__(kThreads, 1) apsp_sym_kernel(const ApspArgs a,
           uint4* const hi = level + tri_base(i);
           unsigned cd = 0, co = 0;
           sym_sweep<R, false>(s, from, dst, hi, a.adj, N, d, a.vec4, first, next, li, (early >> L) & 1u,
-                              warp_id, n_warps, cd, co);
+                              warp_id, n_warps, cd, co, full);
           sym_add((unsigned long long)cd + 2ull * co, s_acc + L);
           grid_arrive(ctrl);
           if (L == kSymFirst) finish(i - 1, done);
