@@ -665,6 +665,9 @@ int collect(ggb_batch* b, cudaStream_t st, ggb_result* res) {
     if ((rc = check_team(b->h_ctrl[t], b->team_list.data(), b->team_start[t], b->team_start[t + 1]))) return rc;
   for (int t = 0; t < 2 * b->l_teams; ++t) {
     const int k = t % b->l_teams;
+    // (a level-by-level team names the graph; those left to the windows are undone as well)
+    if (t < b->l_teams && b->h_lctrl[t].error == ggb::kErrAdj)
+      return report(ggb::kErrAdj, 0, b->h_lctrl[t].error_info);
     if ((rc = check_team(b->h_lctrl[t], b->l_list.data(), b->l_start[k], b->l_start[k + 1]))) return rc;
   }
   for (int i = 0; i < b->n; ++i)

@@ -32,13 +32,15 @@ namespace ggb {
 
 constexpr unsigned kLevelsList = 1u << 18;     // listed pairs per team
 constexpr unsigned kLevelsTarget = 1u << 14;   // pairs expected when the last sweep is chosen
-constexpr int kLevelsCounters = 3 * (2 + kSymPasses);   // per team: three sets (list_n, pairs left after each pass)
+constexpr int kLevelsSet = 2 + kSymPasses;       // counters of a graph: list_n, pairs left after each pass, flags
+constexpr int kLevelsFlags = 1 + kSymPasses;     // of them the flags: 1 asymmetric, 2 an id out of range
+constexpr int kLevelsCounters = 3 * kLevelsSet;  // per team: three sets in rotation
 
 enum : int { kLevelsFailed = 0, kLevelsDone = 1, kLevelsNotServed = 2 };
 
 // Per-team workspace of the list.
 struct LevelsList {
-  unsigned* counters;           // [3][2 + kSymPasses], zeroed before the launch
+  unsigned* counters;           // [3][kLevelsSet], zeroed before the launch
   unsigned long long* list;     // [kLevelsList]
   unsigned long long* hash;     // [2 * kLevelsList]
   unsigned char* hlev;          // [2 * kLevelsList]
@@ -218,16 +220,23 @@ __device__ __forceinline__ void levels_transposes(uint4* m, int N, int C, long l
 
 // One graph on the `ncta` CTAs of a team (this one is number `cta`), as
 // eval_windows: m0 and m1 are its two matrices of N rows of levels_pitch(N)
-// uint4; `turn` counts the team's graphs.  kLevelsFailed: a wait ran out or an
-// error was reported, the caller leaves the kernel.
-__device__ __forceinline__ int eval_levels(const ApspArgs& a, const LevelsList& ws, unsigned turn, uint4* m0, uint4* m1,
+// uint4; `turn` counts the team's graphs, `name` stands for this one in an
+// error.  kLevelsFailed: a wait ran out or an error was reported, the caller
+// leaves the kernel.
+//
+// A CTA that is done with a graph goes on to the team's next one without a
+// barrier, so nothing the next graph's seeding writes may be read late for this
+// one: what a graph's CTAs tell one another lies in its own set of counters.  A
+// set is cleared in the graph before its use, two after its last readers, whose
+// CTAs have all arrived at a barrier since.
+__device__ __forceinline__ int eval_levels(const ApspArgs& a, const LevelsList& ws, unsigned turn, int name, uint4* m0, uint4* m1,
                                            int cta, int ncta, ApspSmem& sm, unsigned* s_dyn,
                                            unsigned long long& bar_target, unsigned& gl, EvalOut& out) {
   const int N = a.N, d = a.d, C = levels_pitch(N);
   const int warp = threadIdx.x >> 5;
   const long long warp_id = (long long)cta * kWarps + warp, n_warps = (long long)ncta * kWarps;
   ApspCtrl* const ctrl = a.ctrl;
-  unsigned* const set = ws.counters + (turn % 3) * (2 + kSymPasses);
+  unsigned* const set = ws.counters + (turn % 3) * kLevelsSet;
   SymArgs s;
   s.list_n = set;
   s.list = ws.list;
@@ -237,10 +246,8 @@ __device__ __forceinline__ int eval_levels(const ApspArgs& a, const LevelsList& 
     bar_target += (unsigned)ncta;
     return grid_barrier(ctrl, bar_target, a.timeout_ns, &sm.flag);
   };
-  // the set of counters the team's next graph uses (its last readers are two graphs back)
   if (cta == 0)
-    for (int i = threadIdx.x; i < 2 + kSymPasses; i += blockDim.x)
-      ws.counters[((turn + 1) % 3) * (2 + kSymPasses) + i] = 0u;
+    for (int i = threadIdx.x; i < kLevelsSet; i += blockDim.x) ws.counters[((turn + 1) % 3) * kLevelsSet + i] = 0u;
   long long sum = 0, prev_total = N, dense = 0;
   int kk = 0, act = 0;
   // ---- S_1 and S_2 -----------------------------------------------------------------
@@ -252,17 +259,19 @@ __device__ __forceinline__ int eval_levels(const ApspArgs& a, const LevelsList& 
       levels_seed<4>(a.adj, N, d, m0, C, s_row, warp_id, n_warps, c, bad, asym);
     else
       levels_seed<1>(a.adj, N, d, m0, C, s_row, warp_id, n_warps, c, bad, asym);
-    if (bad) set_error(ctrl, kErrAdj, (int)blockIdx.x);
-    if (asym) ctrl->asym = (int)turn + 1;
+    if (bad) set_error(ctrl, kErrAdj, name);
+    const unsigned flags = __reduce_or_sync(0xffffffffu, (bad ? 2u : 0u) | (asym ? 1u : 0u));
+    if ((threadIdx.x & 31) == 0 && flags) atomicOr(set + kLevelsFlags, flags);
     cta_add_counts<4>(c, ctrl, gl, sm.red);
   }
   if (!barrier()) return kLevelsFailed;
   read_level_counts(ctrl, gl, 2, sm.seen, sm.lvl);
   const long long c1 = sm.lvl[0], c2 = sm.lvl[2];
   __syncthreads();
-  if (ld_volatile_i32(&ctrl->error) != 0) return kLevelsFailed;
   gl += 2;
-  if (ld_volatile_i32(&ctrl->asym) == (int)turn + 1) return kLevelsNotServed;
+  const unsigned flags = __ldcg(set + kLevelsFlags);
+  if (flags & 2u) return kLevelsFailed;
+  if (flags & 1u) return kLevelsNotServed;
   act = level_decision(1, c1, 0, N, N, N, 0, 1, prev_total, sum);
   if (!act) {
     kk = 1;
@@ -289,7 +298,6 @@ __device__ __forceinline__ int eval_levels(const ApspArgs& a, const LevelsList& 
     read_level_counts(ctrl, gl, 1, sm.seen, sm.lvl);
     const long long total = sm.lvl[0] + 2 * sm.lvl[1];
     __syncthreads();
-    if (ld_volatile_i32(&ctrl->error) != 0) return kLevelsFailed;
     ++gl;
     ++dense;
     if (last) {
@@ -340,7 +348,7 @@ static __global__ void __launch_bounds__(kThreads, 1) apsp_levels_kernel(const A
   unsigned long long bar_target = 0;
   unsigned gl = 0;
   EvalOut o;
-  const int r = eval_levels(a, ws, 0u, a.buf0, a.buf1, (int)blockIdx.x, (int)gridDim.x, sm, s_dyn, bar_target, gl, o);
+  const int r = eval_levels(a, ws, 0u, (int)blockIdx.x, a.buf0, a.buf1, (int)blockIdx.x, (int)gridDim.x, sm, s_dyn, bar_target, gl, o);
   if (r == kLevelsFailed || blockIdx.x != 0 || threadIdx.x != 0) return;
   ApspCtrl* c = a.ctrl;
   if (r == kLevelsNotServed) {
@@ -393,7 +401,7 @@ static __global__ void __launch_bounds__(kThreads, 1) apsp_batch_levels_kernel(c
     a.d = gr.d;
     a.vec4 = gr.vec4;
     EvalOut o;
-    const int r = eval_levels(a, ws, (unsigned)(k - k0), m0, m1, cta, b.team_ctas, sm, s_dyn, bar_target, gl, o);
+    const int r = eval_levels(a, ws, (unsigned)(k - k0), gi, m0, m1, cta, b.team_ctas, sm, s_dyn, bar_target, gl, o);
     if (r == kLevelsFailed) {
       if (b.sticky && threadIdx.x == 0) atomicCAS(b.sticky, 0, max(1, ld_volatile_i32(&a.ctrl->error)));
       return;
