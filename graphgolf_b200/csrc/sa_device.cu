@@ -599,7 +599,8 @@ __global__ void decide_kernel(State* __restrict__ s, const Swap* __restrict__ sw
                               const BatchOut* __restrict__ out, int K, const Swap* __restrict__ comp,
                               const BatchOut* __restrict__ comp_out, float* __restrict__ labels,
                               const Swap* __restrict__ pred, int C) {
-  if (s->done) return;
+  if (s->done) return;   // read by every thread before thread 0 can set it
+  __syncthreads();
   decide_step(s, sw, sel, out, K, comp, comp_out, labels, pred, C);
 }
 
@@ -612,7 +613,7 @@ __global__ void decide_kernel(State* __restrict__ s, const Swap* __restrict__ sw
 constexpr int kPlainLines = 16384;
 __global__ void __launch_bounds__(512) plain_step_kernel(State* __restrict__ s, Swap* __restrict__ sw,
                                                          const BatchOut* __restrict__ out) {
-  if (s->done) return;   // read by every thread before thread 0 can set it (the barriers of decide_step)
+  if (s->done) return;   // read by every thread before thread 0 can set it
   __syncthreads();
   if (threadIdx.x == 0) {
     s->prev_total = s->cur_total;
