@@ -801,7 +801,9 @@ int create(int n_graphs, const int* nodes, const int* based_nodes, const int* gr
   if ((rc = dev_alloc(&b->d_tcells, mt))) return rc;
   if ((rc = dev_alloc(&b->d_tsoff, mt))) return rc;
   if ((rc = dev_alloc(&b->d_records, (size_t)n_graphs)) || (rc = dev_alloc(&b->d_lctrl, 2 * mt))) return rc;
-  BCUDA(cudaMemset(b->d_records, 0, (size_t)n_graphs * sizeof(ggb::ApspCtrl)));
+  // set_plan below waits for b->stream, so these come before any launch and upload
+  BCUDA(cudaMemsetAsync(b->d_records, 0, (size_t)n_graphs * sizeof(ggb::ApspCtrl), b->stream));
+  BCUDA(cudaMemsetAsync(b->d_adj, 0, std::max<size_t>((size_t)b->adj_ints, 1) * sizeof(int), b->stream));
   BCUDA(cudaHostAlloc(&b->h_lctrl, 2 * mt * sizeof(ggb::ApspCtrl), cudaHostAllocDefault));
   BCUDA(cudaHostAlloc(&b->h_out, (size_t)n_graphs * sizeof(ggb::BatchOut), cudaHostAllocDefault));
   BCUDA(cudaHostAlloc(&b->h_ctrl, mt * sizeof(ggb::ApspCtrl), cudaHostAllocDefault));
@@ -818,7 +820,6 @@ int create(int n_graphs, const int* nodes, const int* based_nodes, const int* gr
     gs[i].win_bits = 0;
   }
   BCUDA(cudaMemcpy(b->d_graphs, gs.data(), gs.size() * sizeof(ggb::BatchGraph), cudaMemcpyHostToDevice));
-  BCUDA(cudaMemset(b->d_adj, 0, std::max<size_t>((size_t)b->adj_ints, 1) * sizeof(int)));
   return ggb_batch_set_plan(b, 0, 0);
 }
 

@@ -279,7 +279,9 @@ int ensure_ready(int device) {
   CUDA_TRY(cudaFuncSetAttribute((const void*)ggb::ball_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 smem_optin - 4096));
   CUDA_TRY(cudaMalloc(&g.d_sctrl, sizeof(ApspCtrl)));
-  CUDA_TRY(cudaMemset(g.d_sctrl, 0, sizeof(ApspCtrl)));
+  // g.stream does not wait for the legacy stream, and launches may use others
+  CUDA_TRY(cudaMemsetAsync(g.d_sctrl, 0, sizeof(ApspCtrl), g.stream));
+  CUDA_TRY(cudaStreamSynchronize(g.stream));
   CUDA_TRY(cudaHostAlloc(&g.h_sout, sizeof(ApspCtrl), cudaHostAllocDefault));
   for (const void* k : {slice_kernel_for(1), slice_kernel_for(2), (const void*)ggb::slice_push_kernel})
     CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - kSliceStatic));
@@ -550,7 +552,7 @@ int launch_lattice(bool ids16, bool with_deg, int N, int d, int n_src1, int grou
   if (rc) return rc;
   if (!g.d_diff) {   // differences (zero between launches), then the height
     CUDA_TRY(cudaMalloc(&g.d_diff, (ggb::kSliceMaxN / 32 + 1) * sizeof(unsigned)));
-    CUDA_TRY(cudaMemset(g.d_diff, 0, (ggb::kSliceMaxN / 32 + 1) * sizeof(unsigned)));
+    CUDA_TRY(cudaMemsetAsync(g.d_diff, 0, (ggb::kSliceMaxN / 32 + 1) * sizeof(unsigned), st));
   }
   int* const height = reinterpret_cast<int*>(g.d_diff + ggb::kSliceMaxN / 32);
   uint16_t* const rows = reinterpret_cast<uint16_t*>(g.d_packed);

@@ -1413,13 +1413,13 @@ int create(ggb_sa* a, int nodes, int degree, int groups, const int* edges, int K
       (rc = sdev(&a->d_X, GK * ggb::mlp::kFeatures)) || (rc = sdev(&a->d_stats, (size_t)nodes * ggb::kStatLevels)) ||
       (rc = sdev(&a->d_pctrl, 1)) || (rc = sdev(&a->d_sticky, 1)))
     return rc;
-  SCUDA(cudaMemset(a->d_sticky, 0, sizeof(int)));
+  SCUDA(cudaMemsetAsync(a->d_sticky, 0, sizeof(int), a->st));
   SCUDA(cudaMemcpy(a->d_edges, edges, L2 * sizeof(int), cudaMemcpyHostToDevice));
   SCUDA(cudaMemcpy(a->d_best_edges, edges, L2 * sizeof(int), cudaMemcpyHostToDevice));
   SCUDA(cudaMemcpy(a->d_adj, adj.data(), adj.size() * sizeof(int), cudaMemcpyHostToDevice));
-  SCUDA(cudaMemset(a->d_vmark, 0, ((size_t)nodes / 32 + 1) * sizeof(unsigned)));
-  SCUDA(cudaMemset(a->d_swaps, 0, GK * sizeof(Swap)));
-  SCUDA(cudaMemset(a->d_X, 0, GK * ggb::mlp::kFeatures * sizeof(__nv_bfloat16)));
+  SCUDA(cudaMemsetAsync(a->d_vmark, 0, ((size_t)nodes / 32 + 1) * sizeof(unsigned), a->st));
+  SCUDA(cudaMemsetAsync(a->d_swaps, 0, GK * sizeof(Swap), a->st));
+  SCUDA(cudaMemsetAsync(a->d_X, 0, GK * ggb::mlp::kFeatures * sizeof(__nv_bfloat16), a->st));
   // profile window: the widest of 2048 / 4096 / 8192 sources whose two matrices fit in about half the L2
   a->pR = 16;
   for (int R = 64; R >= 16; R /= 2)
