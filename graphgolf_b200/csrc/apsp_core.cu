@@ -146,7 +146,10 @@ struct State {
   unsigned char* h_team = nullptr;   // pinned: the above for upload, then results for read-back
   int last_teams = 0;
   // shared-memory windows (apsp_slice.cuh)
-  ApspCtrl* d_sctrl = nullptr;       // all zero between launches
+  ApspCtrl* d_sctrl = nullptr;       // all zero between launches, see open_record()
+  bool slice_open = false;           // a launch on slice_stream has not been collected
+  cudaStream_t slice_stream = nullptr;
+  bool clear_sctrl = false;          // launches may have overlapped
   ApspCtrl* h_sout = nullptr;        // pinned: the result record the kernel writes
   unsigned* d_packed = nullptr; size_t cap_packed = 0;   // the 16-bit rows of a lattice
   unsigned* d_diff = nullptr;        // lattice_prep_kernel's differences and the height
@@ -480,6 +483,30 @@ SlicePlan plan_slice(int N, int d, int n_src1, int ac) {
   return p;
 }
 
+// Before a shared-memory launch on st: no result of an earlier one is left in the
+// record, and the control block counts this launch's CTAs from zero.  A
+// launch's last CTA leaves the control block clear, which is enough (and 2 us
+// less a call) while launches follow one another.  Launches on different streams
+// may overlap and spoil one another's results, but not those of later calls: once
+// that can have happened -- an uncollected launch on another stream, or a captured
+// one, whose replays are not seen here -- every launch clears the block first.
+int open_record(cudaStream_t st) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  CUDA_TRY(cudaStreamIsCapturing(st, &capturing));
+  const bool captured = capturing != cudaStreamCaptureStatusNone;
+  if (captured || (g.slice_open && g.slice_stream != st)) g.clear_sctrl = true;
+  if (g.clear_sctrl) CUDA_TRY(cudaMemsetAsync(g.d_sctrl, 0, sizeof(ApspCtrl), st));
+  if (captured) {
+    CUDA_TRY(cudaMemcpyAsync(g.h_sout, g.d_sctrl, sizeof(ApspCtrl), cudaMemcpyDeviceToHost, st));
+  } else {
+    g.h_sout->done = 0;
+    g.h_sout->error = 0;
+  }
+  g.slice_open = true;
+  g.slice_stream = st;
+  return GGB_OK;
+}
+
 void launched_slices(int N, int width) {
   g.ev_ball = false;
   g.last_N = N;
@@ -522,6 +549,8 @@ int launch_slice(const SlicePlan& pl, const int* d_adj, const uint16_t* d_adj16,
   a.adj = d_adj;
   a.adj16 = d_adj16;
   a.deg = deg;
+  int rc = open_record(st);
+  if (rc) return rc;
   if (g.timing) CUDA_TRY(cudaEventRecord(g.ev[0], st));
   if (g.timing) CUDA_TRY(cudaEventRecord(g.ev[1], st));
   if (pl.words == 1)
@@ -549,7 +578,7 @@ int launch_lattice(bool ids16, bool with_deg, int N, int d, int n_src1, int grou
   ggb::SliceArgs a = slice_args(N, d, n_src1, N, 0, groups, width);
   const size_t row_words = ((size_t)N * a.dp + 1) / 2;
   int rc = grow_device(&g.d_packed, &g.cap_packed, row_words);
-  if (rc) return rc;
+  if (rc || (rc = open_record(st))) return rc;
   if (!g.d_diff) {   // differences (zero between launches), then the height
     CUDA_TRY(cudaMalloc(&g.d_diff, (ggb::kSliceMaxN / 32 + 1) * sizeof(unsigned)));
     CUDA_TRY(cudaMemsetAsync(g.d_diff, 0, (ggb::kSliceMaxN / 32 + 1) * sizeof(unsigned), st));
@@ -974,6 +1003,7 @@ int read_ctrl(cudaStream_t st, ggb_partial* p) {
     CUDA_TRY(cudaMemcpyAsync(g.h_ctrl, g.d_ctrl, (g.last_sym ? 2 : 1) * sizeof(ApspCtrl), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
   g.pending = false;
+  if (st == g.slice_stream) g.slice_open = false;
   const ApspCtrl& c = g.last_slice ? *g.h_sout : g.h_ctrl[g.last_sym && g.h_ctrl[0].fallback ? 1 : 0];
   if (c.error == ggb::kErrAdj)
     return fail(GGB_EADJ, "adjacency entry outside [0, nodes) (reported by CTA/vertex %d)", c.error_info);
@@ -984,7 +1014,7 @@ int read_ctrl(cudaStream_t st, ggb_partial* p) {
   if (c.error == ggb::kErrDegree)
     return fail(GGB_EINVAL, "degree of vertex %d outside [0, max_degree]", c.error_info);
   if (c.error != 0) return fail(GGB_ECUDA, "device error code %d", c.error);
-  if (!c.done) return fail(GGB_ECUDA, "the persistent kernel did not complete");
+  if (!c.done) return fail(GGB_ECUDA, "the evaluation did not complete");
   p->diam = c.diam;
   p->disconnected = c.disconnected;
   p->sum = c.sum;
