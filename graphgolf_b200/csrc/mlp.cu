@@ -906,6 +906,7 @@ int ggb_mlp_time_forward(ggb_mlp* m, const float* x, int rows, int reps, double*
     return core_fail(GGB_EINVAL, "rows must be a multiple of 16 up to max_rows, reps positive");
   int rc = upload_x(m, x, rows);
   if (rc) return rc;
+  MCUDA(cudaStreamSynchronize(nullptr));   // the timing stream below does not wait for the upload's
   cudaStream_t st = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);

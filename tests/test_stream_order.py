@@ -12,3 +12,11 @@ def test_fills_name_their_stream(name):
     text = (build.CSRC / name).read_text()
     assert "cudaStreamNonBlocking" in text
     assert not re.findall(r"cudaMemset(?:2D)?\s*\(", text)
+
+
+def test_timed_forward_waits_for_its_upload():
+    """The features are cast on the legacy stream, the forwards run on another."""
+    text = (build.CSRC / "mlp.cu").read_text()
+    body = text[text.index("int ggb_mlp_time_forward("):]
+    upload, stream = body.index("upload_x("), body.index("cudaStreamCreateWithFlags")
+    assert upload < body.index("cudaStreamSynchronize(nullptr)") < stream
