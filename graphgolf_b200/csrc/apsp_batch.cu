@@ -562,7 +562,7 @@ int launch(ggb_batch* b, cudaStream_t st, bool use_graph) {
   }
   BCUDA(cudaEventRecord(b->ev[1], st));
   b->timed = 1;
-  ggb::core_add_launches(1);
+  ggb::core_add_launches(b->kernels());
   b->pending = true;
   return GGB_OK;
 }
@@ -622,7 +622,7 @@ int eval_parts(ggb_batch* b, const int* const* adj) {
     BCUDA(cudaEventRecord(b->ev[2 * b->timed + 1], b->stream));
     b->timed += 1;
   }
-  ggb::core_add_launches(1);
+  ggb::core_add_launches(b->kernels());
   b->pending = true;
   return GGB_OK;
 }

@@ -78,6 +78,9 @@ struct ggb_batch {
   // (device; only while every graph is on slices, see all_slices).
   const int* patch_base = nullptr;
   const ggb::Swap* patch = nullptr;
+  // Kernels of one evaluation: the level-by-level launch and the windows behind
+  // it, the window teams, the slices.
+  int kernels() const { return (l_teams > 0 ? 2 : 0) + (n_teams > 0 ? 1 : 0) + (int)slices.size(); }
   bool all_slices() const { return split && l_teams == 0 && n_teams == 0 && !slice_items.empty(); }
   const int* stop = nullptr;         // device flag: the launch does nothing while it is non-zero
   int* sticky = nullptr;             // device flag: first error code of any launch (set, never cleared)

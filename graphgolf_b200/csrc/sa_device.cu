@@ -1083,7 +1083,7 @@ int enqueue_step(ggb_sa* a, cudaStream_t st) {
     int rc = ggb::batch_enqueue(a->cand, st);
     if (rc) return rc;
     plain_step_kernel<<<1, 512, 0, st>>>(s, a->d_swaps, a->cand->d_out);
-    ggb::core_add_launches(2);
+    ggb::core_add_launches(1 + a->cand->kernels());
     SCUDA(cudaGetLastError());
     return GGB_OK;
   }
@@ -1123,6 +1123,7 @@ int enqueue_step(ggb_sa* a, cudaStream_t st) {
     }
     rc = ggb::batch_enqueue(a->cand, st);
     if (rc) return rc;
+    launches += a->cand->kernels();
     singles = a->cand->d_out;
   }
   compose_kernel<<<1, kComposeThreads, 0, st>>>(s, a->d_swaps, sel, singles, a->K, a->d_comp, a->compose_max,
@@ -1143,7 +1144,7 @@ int enqueue_step(ggb_sa* a, cudaStream_t st) {
     rc = ggb::batch_enqueue(a->comp, st);
     if (rc) return rc;
     comp_out = a->comp->d_out;
-    launches += 2;
+    launches += 2 + a->comp->kernels();
   }
   decide_kernel<<<1, std::max(32, (a->K + 31) / 32 * 32), 0, st>>>(s, a->d_swaps, sel, singles, a->K, a->d_comp,
                                                                    comp_out, a->learned ? a->d_labels : nullptr,
