@@ -608,6 +608,13 @@ int eval_parts(ggb_batch* b, const int* const* adj) {
   for (int r = 0; r < b->n; ++r) end[(int)kind[b->by_size[r]]] = r + 1;
   std::sort(order, order + 3, [&](int x, int y) { return end[x] < end[y]; });
   const int bits[3] = {ggb::kPartSlices, ggb::kPartWindows, ggb::kPartLevels};
+  // a launch that has not been collected may still run on another stream, with
+  // the same adjacencies, workspaces and control blocks (graph launches wait for
+  // one another)
+  if (b->pending) {
+    BCUDA(cudaStreamWaitEvent(b->stream, b->ev[1], 0));
+    BCUDA(cudaStreamWaitEvent(b->copies, b->ev[1], 0));
+  }
   int rc = ggb::batch_enqueue(b, b->stream, ggb::kPartClear), at = 0;
   if (rc) return rc;
   b->timed = 0;
