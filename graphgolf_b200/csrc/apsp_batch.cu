@@ -365,8 +365,18 @@ int upload_split(ggb_batch* b) {
 
 void model_choice(ggb_batch* b, const std::vector<int>& ids, int* R, int* T);
 
+// No kernels: nothing of a plan whose buffers could not be had is launched.
+void no_plan(ggb_batch* b) {
+  b->slices.clear();
+  b->slice_items.clear();
+  b->slice_words.assign(b->n, 0);
+  b->l_teams = 0;
+  b->n_teams = b->ctas = 0;
+  b->stamp_ints = 0;
+}
+
 // The automatic plan.  Falls back to one windows plan for all graphs when the
-// level-by-level workspace cannot be had.
+// workspace of the other kernels cannot be had.
 int plan_split(ggb_batch* b) {
   drop_graph(b);
   b->split = true;
@@ -407,30 +417,31 @@ int plan_split(ggb_batch* b) {
   plan_levels(b, mid);
   int rc = upload_split(b);
   if (rc == GGB_ENOMEM) {
-    b->l_teams = 0;
-    rest.insert(rest.end(), mid.begin(), mid.end());
+    no_plan(b);
+    rest = all_graphs(b);
     rc = GGB_OK;
   }
-  if (rc) return rc;
   b->n_teams = b->ctas = 0;
   b->stamp_ints = 0;
-  if (rest.empty()) return GGB_OK;
-  int R = 1, T = 1;
-  model_choice(b, rest, &R, &T);
-  make_plan(b, rest, R, T, true);
-  return upload_windows(b);
+  if (!rc && !rest.empty()) {
+    int R = 1, T = 1;
+    model_choice(b, rest, &R, &T);
+    make_plan(b, rest, R, T, true);
+    rc = upload_windows(b);
+  }
+  if (rc) no_plan(b);
+  return rc;
 }
 
 // One windows plan for all graphs.
 int plan_fixed(ggb_batch* b, int R, int T) {
   drop_graph(b);
+  no_plan(b);
   b->split = false;
-  b->slices.clear();
-  b->slice_items.clear();
-  b->slice_words.assign(b->n, 0);
-  b->l_teams = 0;
   make_plan(b, all_graphs(b), R, T, true);
-  return upload_windows(b);
+  const int rc = upload_windows(b);
+  if (rc) no_plan(b);
+  return rc;
 }
 
 ggb::BatchArgs batch_args(const ggb_batch* b) {
@@ -479,7 +490,7 @@ int coop(const void* fn, int ctas, size_t smem, void** params, cudaStream_t st) 
 // (kPartClear, before any part's results are written).
 int ggb::batch_enqueue(ggb_batch* b, cudaStream_t st, int parts) {
   int rc;
-  if ((parts & kPartClear) && (b->l_teams > 0 || b->n_teams > 0))
+  if ((parts & kPartClear) && (b->l_teams > 0 || b->n_teams > 0 || b->slices.empty()))
     BCUDA(cudaMemsetAsync(b->d_out, 0, (size_t)b->n * sizeof(ggb::BatchOut), st));
   if ((parts & kPartLevels) && b->l_teams > 0) {
     const size_t words = ggb::kLevelsListWords + (ggb::kLevelsCounters + 1) / 2;
