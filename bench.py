@@ -147,6 +147,22 @@ def sweep_bytes(nodes: int, degree: int, dense_levels: int, window_bits: int) ->
     return dense_levels * (nodes * degree * 4 + nodes * degree * row + 2 * nodes * row)
 
 
+def half_sweep_bytes(nodes: int, degree: int, dense_levels: int, window_bits: int) -> int:
+    """Algorithmic bytes of the half sweeps of a symmetric graph per launch:
+    window i sweeps the rows from its first source on, every sweep but the last
+    of the windows behind the first writes them, and the rows below are
+    transposes (read once, written once) at every level that is written."""
+    row = window_bits // 8
+    windows = -(-nodes // window_bits)
+    sweeps = dense_levels // windows
+    total = 0
+    for i in range(windows):
+        rows, writes = nodes - i * window_bits, sweeps - (1 if i else 0)
+        total += rows * (sweeps * (degree * 4 + degree * row + row) + writes * row)
+        total += 2 * writes * (nodes - rows) * row
+    return total
+
+
 def ball_bytes(nodes: int, degree: int, windows: int, window_bits: int) -> int:
     """Algorithmic bytes of the ball pre-pass: the 1 + d + d^2 + d^3 adjacency
     entries of every vertex's three-hop ball read, and its S_3 row of every
@@ -166,6 +182,13 @@ def _profile(workload: str) -> dict:
     workload (profiles/apsp_<workload>_traffic.json), or {}."""
     tp = ROOT / "profiles" / f"apsp_{workload}_traffic.json"
     return json.loads(tp.read_text()) if tp.exists() else {}
+
+
+def captured(prof: dict, kernel: str, window_bits: int) -> dict:
+    """The capture of `kernel` in a profile, if it was taken at this window
+    width, or {}."""
+    k = prof.get(kernel, {})
+    return k if k.get("window_bits") == window_bits else {}
 
 
 def l2_gather_roof(lib, n: int, d: int, window_bits: int):
@@ -224,10 +247,10 @@ def roofline(kernel: str, alg: float, ms: float, l2_roof, hbm_peak: float, hbm_k
             out["frac_of_l2_stream"] = out["lts_gbs"] / l2_stream
     if lts_pct is not None:
         out["lts_throughput_pct"] = lts_pct
-    out["note"] = ("achieved counts every gather of every dense sweep (the reference algorithm's bytes), "
-                   "including the rows that half sweeps take from transposes and the parts that fullness "
-                   "checks and full-row stamps skip, so it can read above the ceiling; frac_of_l2_stream is the physical L2 rate against it; traffic = DRAM "
-                   "bytes per launch from the committed ncu capture under profiles/")
+    out["note"] = ("achieved counts every gather of every row that a dense sweep takes, including the parts that "
+                   "fullness checks and full-row stamps skip, so it can read above the ceiling; frac_of_l2_stream "
+                   "is the physical L2 rate against it; traffic = DRAM bytes per launch from the committed ncu "
+                   "capture of this kernel at this window width under profiles/, null without one")
     return out
 
 
@@ -550,12 +573,13 @@ def main() -> int:
     # dominant kernel: the dense sweeps; the ball pre-pass is reported beside it
     pers_ms = statistics.mean(kt_pers) if kt_pers else mean_ms
     ball_ms = statistics.mean(kt_ball) if kt_ball else 0.0
-    alg = sweep_bytes(n, d, first.dense_levels, first.window_bits)
-    achieved = alg / (pers_ms / 1e3) / 1e9
     l2_roof = l2_gather_roof(lib, n, d, first.window_bits)
     prof = _profile(args.workload)
-    main = "apsp_sym_kernel" if "apsp_sym_kernel" in prof and not args.window_bits else "apsp_persistent_kernel"
-    kp = prof.get(main, {})
+    half = "apsp_sym_kernel" in prof and not args.window_bits
+    main = "apsp_sym_kernel" if half else "apsp_persistent_kernel"
+    alg = (half_sweep_bytes if half else sweep_bytes)(n, d, first.dense_levels, first.window_bits)
+    kp = captured(prof, main, first.window_bits)
+    kb = captured(prof, "sym_ball_kernel" if half else "ball_kernel", first.window_bits)
     traffic = kp.get("dram_bytes_per_launch")
     lts = kp.get("lts_bytes_per_launch")
 
@@ -573,8 +597,7 @@ def main() -> int:
             "ball_prepass": {"ms_per_launch": ball_ms,
                              "algorithmic_bytes_per_launch": ball_bytes(n, d, first.windows, first.window_bits)
                              if ball_ms else 0,
-                             "traffic": prof.get("sym_ball_kernel" if main == "apsp_sym_kernel" else "ball_kernel",
-                                                 {}).get("dram_bytes_per_launch")},
+                             "traffic": kb.get("dram_bytes_per_launch")},
             "survey_formula_bytes_per_eval": survey_formula_bytes(n, d, first.levels, first.window_bits),
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d_per_step),
                     "d2h_bytes_per_step": 96, "input_bytes_per_step": n * d * 4,
@@ -721,6 +744,9 @@ def batch_bench(peak: float, peak_kind: str, lib) -> dict:
               else f"apsp_batch_kernel<{bits // 128}>")
     roof = roofline(kernel, alg, kms, l2, peak, peak_kind, None, None,
                     l2_stream=l2_stream_roof(lib))
+    if mixed:
+        roof["note"] += ("; counts whole sweeps of every graph, of which the level-by-level teams gather the lower "
+                         "triangle and the shared-memory windows nothing through L2")
     roof["l2_gather_probe_case"] = "N=16384, d=12: the largest graphs of the batch"
     return {"workload": "4096-vertex base + 256 single-swap candidates, d=12, N log-uniform 512..16384",
             "graphs": len(w), "plan": {"window_bits": bits, "team_ctas": team, "autotune_s": tune_s},
