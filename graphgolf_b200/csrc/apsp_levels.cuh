@@ -22,9 +22,17 @@
 // is left to eval_windows (kLevelsNotServed).
 //
 // Bound: the latency of a task's chain (ids, then two groups of eight gathers)
-// and two barriers a level; the gathers run at 5 TB/s on the whole GPU.
+// and two barriers a level: 906 MB through L2 at 6.5 TB/s for N = 16384, d = 12 on
+// the whole GPU, issue slots 31 % busy.
 // Measured, kernel us: N = 16384, d = 12 144 on 148 CTAs (the persistent kernel
 // with its ball 182), 218 on 74, 370 on 37 (467 there), 745 on 16 (948).
+//
+// Graphs that it does not suit, whole call, us, against the persistent kernel:
+// one asymmetric row, d = 8, which costs the seeding, 187 / 169 at N = 12000, 271 / 185
+// at 16000; a random core whose vertices carry a leaf each, rows of 7, where the
+// list overflows and a level is swept twice, 182 / 159 at 8600, 355 / 228 at 12000,
+// 394 / 234 at 16000; two components, d = 8, 136 / 100 at 12000, 171 / 121 at 16000;
+// circulants of 20 to 4000 levels between 15 % faster and 20 % slower.
 #pragma once
 #include "apsp_sym.cuh"
 

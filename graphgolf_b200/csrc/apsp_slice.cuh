@@ -144,10 +144,12 @@ __device__ __forceinline__ void slice_finish(const SliceArgs& a, const SliceTota
 // is full.
 //
 // Bound: at N = 256 the launch, the staging and the record's way out (11 us;
-// the persistent kernel took 37); from N = 1024 on the shared-memory wavefronts
-// of the random row reads, about 3.5 per 32 four-byte reads and 6.2 per 32
-// eight-byte ones (N = 1024, d = 8: 15 us, was 27; N = 4700, d = 6: 39 us, was
-// 48; N = 9000, d = 3: 90 us, was 228).
+// the persistent kernel took 37); from N = 1024 on issue slots (56 to 65 % busy
+// on the SMs with a window) and the shared-memory wavefronts of the random row
+// reads: over all shared loads 2.2 a load with four-byte rows and 3.3 to 3.5 with
+// eight-byte ones, the load/store data pipe 48 % busy at N = 4700, d = 6 and 67 % at
+// N = 9000, d = 3 (N = 1024, d = 8: 15 us, was 27; N = 4700, d = 6: 39 us, was 48;
+// N = 9000, d = 3: 90 us, was 228).
 //
 // Shared memory: two row buffers and the adjacency.
 inline size_t slice_smem_bytes(int np, int words, int pairs) { return (size_t)np * (words * 8 + pairs * 4); }
@@ -326,8 +328,9 @@ __global__ void __launch_bounds__(1024, 1) slice_batch_kernel(const BatchGraph* 
 // 100 x 100 lattice with edges of length 3 changes about 1000 of its 10 000
 // vertices a level.
 //
-// Bound: instructions (about 130 per 32 vertices visited) and the last windows
-// (313 windows of 45 to 78 levels on 148 SMs).  100 x 100, degree 4, length 3:
+// Bound: a level's chain (list entry, row, new bits, pushes, append, barrier: 2.5 us
+// a level; 127 million warp instructions in all, issue slots 49 % busy) and the
+// last windows (313 windows of 45 to 78 levels on 148 SMs).  100 x 100, degree 4, length 3:
 // 347 us with the two preparing kernels, where the persistent kernel took 1305
 // us (79 levels of two windows at a grid barrier each) and slice_kernel 670 us.
 //

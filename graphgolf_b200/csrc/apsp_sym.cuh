@@ -37,15 +37,26 @@
 // Measured (whole call, us, against the persistent kernel with its ball):
 // N = 65536, d = 16 1218 / 1836 (ball 271 / 380, sweeps 910 / 1425); d = 8
 // 1528 / 2312; N = 16384, d = 12 182 / 216; N = 100000, d = 12 3240 / 6930;
-// N = 262144, d = 12 30 900 / 67 900.  Bound: L2 gathers, at 7 to 10 TB/s (the
-// persistent kernel's sweeps reach 13: half of the rows of a level lie in the
-// store, and the ball is read from HBM), and for the ball the load/store pipe
-// (91 % busy).  Tried and not kept: S_3 in halves too (the ball kernel 9 %
+// N = 262144, d = 12 30 900 / 67 900.  Bound: L2 gathers (N = 65536,
+// d = 16: 12.1 GB through L2 at 13.1 TB/s, and 2.4 GB read from HBM, where the
+// ball and part of the store lie), and for the ball the load/store data pipe
+// (92 % busy).  Tried and not kept: S_3 in halves too (the ball kernel 9 %
 // faster, its transposes cost more), sweeps that write every row twice instead
 // of choosing between two places (4 % slower), a prefetch of the next window's
 // ball slice into L2 (2 % slower), windows of 1024 to 2048 sources, 768 or 1024
 // threads with 6 or 4 neighbour rows in flight (10 to 20 % slower), half a warp
 // per 1 KB row with two parts a lane (5 % slower).
+//
+// A graph that is left to the persistent kernel has paid for the ball and the
+// first window, and that kernel runs without a ball of its own.  Whole call, us,
+// against the persistent kernel with its ball, at N = 65536 (and 20000): one
+// asymmetric row, d = 8 2970 / 2290 (361 / 354), d = 12 2810 / 2080 (385 / 314); a
+// random core whose vertices carry a leaf each, rows of 7, 3880 / 3200 (515 /
+// 459); two components, d = 8, which stall in the first window, 657 / 384 (229 /
+// 150).  Circulants of 24 to 334 levels gain by the wider windows at
+// N = 65536 (334 levels 108 / 141 ms) and lose 1 to 10 % at 20000 and 30000.  Warps
+// that stop working once the list is too long changed nothing: the time lies
+// before that.
 #pragma once
 #include "apsp_kernel.cuh"
 
