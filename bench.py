@@ -749,7 +749,8 @@ def batch_bench(peak: float, peak_kind: str, lib) -> dict:
                          "triangle and the shared-memory windows nothing through L2")
     roof["l2_gather_probe_case"] = "N=16384, d=12: the largest graphs of the batch"
     return {"workload": "4096-vertex base + 256 single-swap candidates, d=12, N log-uniform 512..16384",
-            "graphs": len(w), "plan": {"window_bits": bits, "team_ctas": team, "autotune_s": tune_s},
+            "graphs": len(w), "plan": {"automatic": mixed, "best_fixed_window_bits": bits, "best_fixed_team_ctas": team,
+                                      "autotune_s": tune_s},
             "value": len(w) / (kms / 1e3), "unit": "graphs/s", "ms_per_batch": kms,
             "e2e": {"value": len(w) / (e2e_ms / 1e3), "unit": "graphs/s", "ms_per_batch": e2e_ms,
                     "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": 48 * len(w),

@@ -48,6 +48,9 @@ struct ggb_batch {
   // teams (apsp_levels.cuh), the rest on teams of windows as a fixed plan has
   // them all.
   bool split = false;
+  // What ggb_batch_get_plan reports for the automatic plan (0: the cost model's
+  // fixed plan), set by the autotuner
+  int best_fixed_R = 0, best_fixed_T = 0;
   struct SliceLaunch { int words, threads, first, items; size_t smem; };
   std::vector<SliceLaunch> slices;          // by shared memory, so that small graphs share an SM
   std::vector<ggb::SliceItem> slice_items;

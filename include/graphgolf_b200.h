@@ -286,14 +286,16 @@ void ggb_batch_destroy(ggb_batch *b);
 
 /* Fixes the plan: window_bits = 128 * 2^k (<= 4096), team_ctas >= 1; a 0
  * leaves that choice to the cost model, two 0s are the automatic plan.
- * ggb_batch_get_plan reports, for the automatic plan, its window teams, or its
- * level-by-level teams when it has no window teams, or its shared-memory windows. */
+ * ggb_batch_get_plan reports, for the automatic plan, the fixed plan for all
+ * graphs that the cost model would take, or that ggb_batch_autotune found
+ * best: what a caller that keeps a plan can set again (two 0s set the automatic
+ * plan again). */
 int ggb_batch_set_plan(ggb_batch *b, int window_bits, int team_ctas);
 int ggb_batch_get_plan(const ggb_batch *b, int *window_bits, int *team_ctas, int *teams);
 
 /* Times the automatic plan and every feasible (window_bits, team_ctas) pair on
  * the batch's current adjacency (iters timed launches each, after one warm-up) and keeps the
- * fastest; reports it and its time. */
+ * fastest; reports it as ggb_batch_get_plan does, and its time. */
 int ggb_batch_autotune(ggb_batch *b, int iters, int *window_bits, int *team_ctas, double *best_ms);
 
 /* Device address of graph i's [nodes][degree] adjacency inside the batch
