@@ -569,6 +569,51 @@ bool lattice_fits(int N) {
   return slices_allowed() && ggb::slice_push_smem_bytes((N + 31) / 32 * 32) <= (size_t)(g.smem_optin - kSliceStatic);
 }
 
+// Levels to expect of a grid graph, from the lengths of 24 sampled edges: the
+// numbering is x * H + y for some H that divides N, and of all those the
+// lattice's own makes the edges shortest.  Edges spread evenly over lengths up to
+// L have a mean of about 2/3 L, and the diameters of such W x H lattices lie at
+// 1.1 to 1.5 (W + H) / L.  Entries out of range are left to the kernels' checks.
+double lattice_levels(int N, int d, const int* deg, const int* adj, const int* rh) {
+  constexpr int kRows = 12, kSample = 2 * kRows;
+  int a[kSample], b[kSample], n = 0;
+  for (int k = 0; k < kRows; ++k) {
+    const int i = (int)((long long)N * k / kRows), di = deg ? std::min(deg[i], d) : d;
+    for (int e = 0; e < 2 && e < di; ++e) {
+      const int u = adj[(size_t)i * d + (e == 0 ? 0 : di - 1)];
+      if ((unsigned)u >= (unsigned)N || (unsigned)rh[i] >= (unsigned)N || (unsigned)rh[u] >= (unsigned)N) continue;
+      a[n] = rh[i];
+      b[n++] = rh[u];
+    }
+  }
+  double levels = 0.0;
+  long long shortest = LLONG_MAX;
+  for (int q = 1; (long long)q * q <= N; ++q) {
+    if (N % q) continue;
+    for (const int H : {q, N / q}) {
+      long long sum = 0;
+      for (int k = 0; k < n; ++k) sum += std::abs(a[k] / H - b[k] / H) + std::abs(a[k] % H - b[k] % H);
+      if (sum >= shortest) continue;
+      shortest = sum;
+      levels = sum > 0 ? 0.83 * (H + N / H) * n / (double)sum : (double)N;
+    }
+  }
+  return levels;
+}
+
+// Whether rings are thin enough for the windows in shared memory, whose time
+// hardly depends on the edges' length, where the other kernels' falls with the
+// levels.  Whole call, us, rings / the others: 80 x 80, d = 6 length 8 183 / 248,
+// 14 171 / 173, 25 171 / 147; 100 x 100, d = 4 length 14 255 / 425, 25 259 / 312, 60
+// 259 / 244, d = 8 length 14 292 / 488, 25 306 / 334, 60 313 / 219; 120 x 120, d = 6
+// length 8 585 / 851, 14 579 / 552, 25 626 / 370, 60 680 / 234.  The two meet at 9 to
+// 14 expected levels up to 10 000 vertices and at 15 to 22 at 14 400.  While every
+// window has an SM to itself (60 x 60) rings are never slower.
+bool rings_are_thin(int N, int d, const int* deg, const int* adj, const int* rh) {
+  if (N <= 32 * g.sms) return true;
+  return lattice_levels(N, d, deg, adj, rh) >= 12.0 * std::max(1.0, std::pow(N / 1.0e4, 1.25));
+}
+
 // Grid evaluation on shared-memory windows: relabel and pack the rows, check
 // the relabel, read the lattice's height off the numbering, then every window
 // in one launch.  The uploaded ids are in d_adj16 or d_adj, rotate_hash in
@@ -1405,7 +1450,7 @@ int eval_grid_impl(int nodes, int degree, const int* deg, int groups, const int*
   if (deg && (rc = check_degrees("degree", deg, nodes, degree))) return rc;
   const size_t n = (size_t)nodes * degree;
   cudaStream_t st = g.stream;
-  const bool lattice = lattice_fits(nodes);
+  const bool lattice = lattice_fits(nodes) && rings_are_thin(nodes, degree, deg, adj, rotate_hash);
   bool ids16 = false;
   rc = stage_adj(adj, n, nodes, st, lattice ? &ids16 : nullptr);
   if (rc) return rc;
