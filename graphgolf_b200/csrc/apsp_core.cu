@@ -791,9 +791,18 @@ int launch_sym(const SymPlan& pl, const int* d_adj, int N, int d, cudaStream_t s
 // persistent kernel's windows fit best (level by level / persistent kernel):
 // d = 4: 10000 216 / 222, 12000 246 / 236, 13400 266 / 243, 15400 278 / 295;
 // d = 6: 12000 182 / 212, 13400 209 / 195, 15400 207 / 211.
-bool levels_served(int N, int d) {
+// They also lose to windows of 8192 sources, two up to 16 384 vertices, where the list
+// takes one level more to fit: d = 5: 8700 156 / 165, 9000 167 / 165, 9200 176 / 165,
+// 11300 194 / 194 (11800, windows of 4096: 196 / 243); d = 7: 8400 152 / 141, 8600 129
+// / 142.  Rows padded with their own ids (non-regular graphs) take a level or two
+// more: max degree 5: 8400 200 / 193, 9000 216 / 190, 10800 231 / 215 (11800: 219 / 264);
+// 6: 9000 192 / 179, 9700 195 / 190, 12300 233 / 215 (10400: 207 / 228).
+bool levels_served(int N, int d, bool padded) {
+  if (!slices_allowed() || d < 4 || d > 32 || N <= 8192 || N > (d >= 16 ? 22000 : 18000)) return false;
+  const bool wide = N <= 15000 && choose_R(N, d, N) == 64;
+  if (wide && (padded ? d <= 6 : d == 5 && N > 8900)) return false;
   if (d <= 6 && N > 12300 && N <= 15000) return false;
-  return slices_allowed() && d >= 4 && d <= 32 && N > 8192 && N <= (d >= 16 ? 22000 : 18000);
+  return d != 7 || N >= 8600;
 }
 
 int launch_levels(const int* d_adj, int N, int d, cudaStream_t st, bool* done) {
@@ -846,7 +855,8 @@ int launch_levels(const int* d_adj, int N, int d, cudaStream_t st, bool* done) {
 }
 
 int launch_apsp(const int* d_adj, int N, int d, int n_src1, int split, int ac, int groups,
-                int rank, int procs, cudaStream_t st, const int* d_adj2 = nullptr, bool lattice = false) {
+                int rank, int procs, cudaStream_t st, const int* d_adj2 = nullptr, bool lattice = false,
+                bool padded = false) {
   if (procs == 1 && !d_adj2) {
     const SlicePlan pl = plan_slice(N, d, n_src1, ac);
     if (pl.words) return launch_slice(pl, d_adj, nullptr, nullptr, N, d, n_src1, split, ac, groups, st);
@@ -855,7 +865,7 @@ int launch_apsp(const int* d_adj, int N, int d, int n_src1, int split, int ac, i
   g.last_sym = false;
   if (procs == 1 && !d_adj2 && groups == 1 && ac == 0 && n_src1 == N && !lattice) {   // lattices have too many levels
     bool done = false;
-    if (levels_served(N, d)) {
+    if (levels_served(N, d, padded)) {
       int rc = launch_levels(d_adj, N, d, st, &done);
       if (rc || done) return rc;
     }
@@ -1553,7 +1563,7 @@ int ggb_eval_general_nonregular(int nodes, int based_nodes, int groups, int max_
   // phase 1 gathers the padded rows; the added-centre phase gathers whole rows
   // (variants/not_regular_general_graph/evaluation.c:180 vs :226)
   rc = launch_apsp(g.d_adj2, nodes, max_degree, based_nodes, based_nodes * groups, added_centers, groups, 0, 1, st,
-                   added_centers ? g.d_adj : nullptr);
+                   added_centers ? g.d_adj : nullptr, false, true);
   if (rc) return rc;
   ggb_partial p;
   rc = read_ctrl(st, &p);
