@@ -1136,7 +1136,7 @@ int stage_adj(const int* adj, size_t n, int nodes, cudaStream_t st, bool* kept16
 
 // Every degree of a non-regular graph lies in [0, max_degree].
 int check_degrees(const char* what, const int* deg, int nodes, int max_degree) {
-  unsigned bad = 0u;   // (a loop without an exit is vectorised: 1 us for 10 000 vertices, 5 with one)
+  unsigned bad = 0u;   // (a loop without an exit is vectorised: 1.4 us for 10 000 vertices, 4.2 with one)
   for (int i = 0; i < nodes; ++i) bad |= (unsigned)deg[i] > (unsigned)max_degree;
   for (int i = 0; bad && i < nodes; ++i)
     if ((unsigned)deg[i] > (unsigned)max_degree) return fail(GGB_EINVAL, "%s[%d] outside [0, max_degree]", what, i);
