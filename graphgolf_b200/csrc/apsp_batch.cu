@@ -152,26 +152,17 @@ double make_plan(ggb_batch* b, const std::vector<int>& ids, int R, int T, bool k
     pq.push(l);
   }
   // Working set of the teams running at once: each team's adjacency and two
-  // matrices.  Past 60 % of L2 the gathers begin to spill to HBM: a steep price
-  // up to about 8500 vertices (22 graphs of 81 to 8357, d = 16: 464 us with it, 525
-  // without), a mild one above (51 graphs of 8192 to 16384 vertices, R = 32: 3.8 ms on 6
-  // teams of 24 CTAs, 100 MB, 4.4 ms on 18 of 8, 315 MB).
+  // matrices.  Past 60 % of L2 the gathers begin to spill to HBM, at a steep price
+  // (with a mild one for large graphs 64 graphs of 10 000 vertices, d = 3 took 13.6 ms, 8.1
+  // with this one, and 16 of 20 000 12.4, 8.7).
   double ws = 0.0;
-  int largest = 0;
   for (int t = 0; t < n_teams; ++t) {
     long long mx = 0;
-    for (int i : lists[t]) {
-      mx = std::max<long long>(mx, (long long)b->N[i] * (b->d[i] * 4 + 32 * R));
-      largest = std::max(largest, b->N[i]);
-    }
+    for (int i : lists[t]) mx = std::max<long long>(mx, (long long)b->N[i] * (b->d[i] * 4 + 32 * R));
     ws += (double)mx;
   }
   const double l2 = (double)b->l2;
-  if (largest <= 8500) {
-    if (ws > 0.6 * l2) makespan *= 1.0 + 1.5 * std::min(1.0, (ws - 0.6 * l2) / (0.6 * l2));
-  } else if (ws > l2) {
-    makespan *= 1.0 + 0.12 * (ws / l2 - 1.0);
-  }
+  if (ws > 0.6 * l2) makespan *= 1.0 + 1.5 * std::min(1.0, (ws - 0.6 * l2) / (0.6 * l2));
   if (!keep) return makespan;
   b->R = R;
   b->T = T;

@@ -1,0 +1,35 @@
+"""Which kernels the automatic plan takes for batches of equal graphs, on both
+sides of its lines (window_bits: 64 in shared memory, at least n level by level,
+128 to 4096 on window teams), against the single-graph evaluator."""
+import pytest
+
+import graphgolf_b200 as gg
+from graphgolf_b200 import graphs
+
+pytestmark = pytest.mark.gpu
+
+
+def _got(r):
+    return (r.connected, r.diameter, r.aspl, r.total)
+
+
+def _kind(r, n):
+    return "levels" if r.window_bits >= n and r.window_bits > 4096 else "slices" if r.window_bits <= 64 else "windows"
+
+
+def _run(n, d, k):
+    adjs = [graphs.random_regular(n, d, s).adj for s in (1, 2)]
+    want = [_got(gg.evaluate(a)) for a in adjs]
+    with gg.Batch([n] * k, d) as b:
+        res = b.evaluate([adjs[i % 2] for i in range(k)])
+        assert [_got(r) for r in res] == [want[i % 2] for i in range(k)]
+        kinds = {_kind(r, n) for r in res}
+        assert len(kinds) == 1
+        return kinds.pop(), b.plan
+
+
+@pytest.mark.parametrize("n,k", [(10000, 32), (20000, 8)])
+def test_window_teams_stay_near_l2(gpu, n, k):
+    """The teams' matrices of graphs that only windows serve (degree 3)."""
+    kind, (bits, _, teams) = _run(n, 3, k)
+    assert kind == "windows" and teams * n * (12 + 32 * bits // 128) < 160e6
