@@ -130,9 +130,10 @@ int team_count(const ggb_batch* b, int n, int R, int* T) {
 }
 
 // Deals the graphs to the teams (longest first, each to the least loaded
-// team) and returns the modelled makespan; fills the plan arrays when
-// `keep`.
-double make_plan(ggb_batch* b, const std::vector<int>& ids, int R, int T, bool keep) {
+// team); returns the modelled makespan and in *spill the teams' working set over
+// 60 % of L2, from where the gathers begin to spill to HBM, in units of L2.
+double deal(const ggb_batch* b, const std::vector<int>& ids, int R, int T, std::vector<std::vector<int>>* teams,
+            double* spill) {
   const int n_teams = team_count(b, (int)ids.size(), R, &T);
   std::vector<double> cost(b->n);
   for (int i : ids) cost[i] = graph_cost(b->N[i], b->d[i], b->bn[i], R, T);
@@ -141,29 +142,37 @@ double make_plan(ggb_batch* b, const std::vector<int>& ids, int R, int T, bool k
   using Load = std::pair<double, int>;
   std::priority_queue<Load, std::vector<Load>, std::greater<Load>> pq;
   for (int t = 0; t < n_teams; ++t) pq.push({0.0, t});
-  std::vector<std::vector<int>> lists(n_teams);
+  teams->assign(n_teams, {});
   double makespan = 0.0;
   for (int i : order) {
     Load l = pq.top();
     pq.pop();
     l.first += cost[i];
-    lists[l.second].push_back(i);
+    (*teams)[l.second].push_back(i);
     makespan = std::max(makespan, l.first);
     pq.push(l);
   }
-  // Working set of the teams running at once: each team's adjacency and two
-  // matrices.  Past 60 % of L2 the gathers begin to spill to HBM, at a steep price
-  // (with a mild one for large graphs 64 graphs of 10 000 vertices, d = 3 took 13.6 ms, 8.1
-  // with this one, and 16 of 20 000 12.4, 8.7).
+  // the teams running at once: each team's adjacency and two matrices
   double ws = 0.0;
-  for (int t = 0; t < n_teams; ++t) {
+  for (const auto& l : *teams) {
     long long mx = 0;
-    for (int i : lists[t]) mx = std::max<long long>(mx, (long long)b->N[i] * (b->d[i] * 4 + 32 * R));
+    for (int i : l) mx = std::max<long long>(mx, (long long)b->N[i] * (b->d[i] * 4 + 32 * R));
     ws += (double)mx;
   }
-  const double l2 = (double)b->l2;
-  if (ws > 0.6 * l2) makespan *= 1.0 + 1.5 * std::min(1.0, (ws - 0.6 * l2) / (0.6 * l2));
+  *spill = std::max(0.0, ws / (double)b->l2 - 0.6);
+  return makespan;
+}
+
+// Deals the graphs to the teams and returns the modelled makespan with the price
+// of a working set past L2; fills the plan arrays when `keep`.  (The price is steep:
+// with a mild one for large graphs 64 graphs of 10 000 vertices, d = 3 took 13.6 ms, 8.1
+// with this one, and 16 of 20 000 12.4, 8.7.)
+double make_plan(ggb_batch* b, const std::vector<int>& ids, int R, int T, bool keep) {
+  std::vector<std::vector<int>> lists;
+  double spill = 0.0;
+  const double makespan = deal(b, ids, R, T, &lists, &spill) * (1.0 + 1.5 * std::min(1.0, spill / 0.6));
   if (!keep) return makespan;
+  const int n_teams = team_count(b, (int)ids.size(), R, &T);
   b->R = R;
   b->T = T;
   b->n_teams = n_teams;
@@ -288,6 +297,76 @@ void plan_slices(ggb_batch* b, const std::vector<int>& ids) {
   }
 }
 
+void model_choice(ggb_batch* b, const std::vector<int>& ids, int* R, int* T);
+
+// ---- slices or teams -------------------------------------------------------------
+// Two models of the kernels' time in us, for random graphs, fitted to 800 batches of
+// 2 to 256 graphs of 64 to 7000 vertices, equal and mixed, d = 3 to 24, each timed both
+// ways (80 % of the predictions within 15 % for slices, 11 % for teams).  The slices
+// are taken while theirs is under 0.92 of the teams': half a percent behind the
+// best of both on average, 7 % slower than teams at worst, 28 % than slices.  Slices
+// alone took up to 1.7 times as long as teams (64 graphs of 2000 vertices, d = 8: 225
+// us, 147), teams alone up to 4 times as long as slices (200 vertices: 12 us, 42).
+
+// Levels of a random d-regular graph of N vertices: its share q of unreached
+// pairs falls like d (d-1)^(k-1) / N at first, then q -> q^(d-1).
+double expected_levels(int N, int d) {
+  if (d < 3) return N;
+  double lq = std::log(std::max(1e-300, 1.0 - std::min(0.999999, (1.0 + d) / N)));
+  int k = 1;
+  for (; k < 200 && 2.0 * std::log((double)N) + lq > std::log(2.0); ++k)
+    lq = lq < -1e-12 ? lq * (d - 1) : std::log1p(-std::min(0.999999, std::pow(d - 1.0, k) * d / N));
+  return k;
+}
+
+// The slices planned in b: what the windows gather (in fours, and less at high
+// degrees, whose rows are full early), barriers and staging, by how many CTAs share
+// an SM; the last window, and the launch.
+double slices_us(const ggb_batch* b) {
+  constexpr double kGather[3] = {1.9e-4, 1.5e-4, 0.73e-4}, kLevel[3] = {0.035, 0.0, 1.46};
+  double us = 0.0;
+  for (const auto& l : b->slices) {
+    const int k = l.smem <= 72 * 1024 ? 0 : l.smem <= 110 * 1024 ? 1 : 2;
+    const double share = std::min((double)(3 - k), std::max(1.0, (double)l.items / b->sms));
+    double sum = 0.0, last = 0.0;
+    for (int t = l.first; t < l.first + l.items; ++t) {
+      const auto& it = b->slice_items[t];
+      const int N = b->N[it.graph], pairs = (b->d[it.graph] + 1) / 2, windows = it.end - it.first;
+      const double levels = expected_levels(N, b->d[it.graph]);
+      const double row = (levels - 1.0) * std::pow(4.0 * ((pairs + 1) / 2), 0.7) + 0.5 * levels * pairs;
+      const double gathers = windows * N * row * (l.words == 1 ? 0.6 : 1.0);
+      sum += gathers * kGather[k] + windows * levels * kLevel[k] + 4.6e-4 * N * pairs;
+      last = std::max(last, gathers * 2.5e-5 * share + 0.23 * windows * levels);
+    }
+    us += sum / b->sms + last + 9.2;
+  }
+  return us;
+}
+
+// The graphs of ids on window teams, as the cost model would plan them: the
+// gathered bytes (rows of 64 bytes and less are slower, and high degrees skip more of them),
+// barriers, seeding (slower where rows are not a multiple of four ids), and the gathers
+// that spill out of L2.
+double windows_us(ggb_batch* b, const std::vector<int>& ids) {
+  int R = 1, T = 1;
+  model_choice(b, ids, &R, &T);
+  std::vector<std::vector<int>> teams;
+  double spill = 0.0, us = 0.0;
+  deal(b, ids, R, T, &teams, &spill);
+  team_count(b, (int)ids.size(), R, &T);
+  for (const auto& team : teams) {
+    double gathers = 0.0, rest = 0.0;
+    for (int i : team) {
+      const double N = b->N[i], d = std::max(b->d[i], 1), levels = expected_levels(b->N[i], b->d[i]);
+      const double windows = std::ceil(b->bn[i] / (128.0 * R));
+      gathers += windows * (levels - 1.0) * N * (std::pow(d, 0.7) + 2.0) * 16.0 * R / T;
+      rest += windows * (3.0 * levels + 1.1 + (b->d[i] % 4 ? 1.3e-4 : 4.4e-5) * N * (d + d * d) * 4.0 / T);
+    }
+    us = std::max(us, gathers * ((R <= 4 ? 2.4e-5 : 1.5e-5) + 1.9e-4 * std::min(spill, 2.0)) + rest);
+  }
+  return us + 9.5;
+}
+
 // Level-by-level teams for the graphs of `ids`: the team size with the least
 // modelled makespan.
 void plan_levels(ggb_batch* b, const std::vector<int>& ids) {
@@ -359,8 +438,6 @@ int upload_split(ggb_batch* b) {
   return GGB_OK;
 }
 
-void model_choice(ggb_batch* b, const std::vector<int>& ids, int* R, int* T);
-
 // No kernels: nothing of a plan whose buffers could not be had is launched.
 void no_plan(ggb_batch* b) {
   b->slices.clear();
@@ -379,9 +456,8 @@ int plan_split(ggb_batch* b) {
   b->best_fixed_R = b->best_fixed_T = 0;
   b->slice_words.assign(b->n, 0);
   // Slices: as for a single graph (plan_slice in apsp_core.cu) while every
-  // window has an SM to itself; with more windows than that they only pay for
-  // smaller graphs (102 graphs of 512 to 3460 vertices, d = 12: 401 us, 393 on
-  // teams; 65 of 256 to 4096, d = 8: 162 / 219; 64 of 1024, d = 8: 52 / 61).
+  // window has an SM to itself; with more windows than that up to fewer gathers a
+  // level, and where slices_us and windows_us say so.
   // Level by level: from 8193 vertices like a single graph; with teams enough
   // to hide its barriers from 4500 (52 graphs of 4096 to 8192 vertices, d = 12:
   // 1198 us, 1309 from 6000 on, 1462 as windows).
@@ -411,6 +487,13 @@ int plan_split(ggb_batch* b) {
     small.clear();
   }
   plan_slices(b, small);
+  long long windows = 0;
+  for (int i : small) windows += (b->bn[i] + 63) / 64;
+  if (windows > 2LL * b->sms && slices_us(b) > 0.92 * windows_us(b, small)) {
+    rest.insert(rest.end(), small.begin(), small.end());
+    plan_slices(b, {});
+    b->slice_words.assign(b->n, 0);
+  }
   plan_levels(b, mid);
   int rc = upload_split(b);
   if (rc == GGB_ENOMEM) {

@@ -28,6 +28,15 @@ def _run(n, d, k):
         return kinds.pop(), b.plan
 
 
+@pytest.mark.parametrize("n,d,k,kind", [(500, 8, 256, "slices"), (2000, 8, 8, "slices"), (2000, 8, 64, "windows"),
+                                        (2000, 5, 64, "windows"), (1000, 16, 64, "windows"), (4000, 5, 32, "windows"),
+                                        (4600, 5, 64, "slices"), (200, 12, 64, "slices"), (64, 2, 40, "slices")])
+def test_small_graphs(gpu, n, d, k, kind):
+    """Windows of 2048 and 4096 sources fit some sizes so well that teams beat
+    one window a CTA."""
+    assert _run(n, d, k)[0] == kind
+
+
 @pytest.mark.parametrize("n,k", [(10000, 32), (20000, 8)])
 def test_window_teams_stay_near_l2(gpu, n, k):
     """The teams' matrices of graphs that only windows serve (degree 3)."""
