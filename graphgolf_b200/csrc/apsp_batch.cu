@@ -460,7 +460,10 @@ int plan_split(ggb_batch* b) {
   // level, and where slices_us and windows_us say so.
   // Level by level: from 8193 vertices like a single graph; with teams enough
   // to hide its barriers from 4500 (52 graphs of 4096 to 8192 vertices, d = 12:
-  // 1198 us, 1309 from 6000 on, 1462 as windows).
+  // 1198 us, 1309 from 6000 on, 1462 as windows).  Degree 4 has more levels, and
+  // windows of 4096 sources fit some sizes well (level by level / windows, 64 graphs): 7000
+  // 3103 / 2807, 8000 3696 / 2864, 8600 4139 / 6500, 9000 5081 / 7150, 10000 5843 /
+  // 5435, 11000 6905 / 7870.
   long long w32 = 0;
   int over = 0;
   for (int i = 0; i < b->n; ++i) {
@@ -476,6 +479,12 @@ int plan_split(ggb_batch* b) {
     if ((long long)N * (d + 1) <= most && N <= ggb::kSliceMaxN && smem <= kSliceSmemMax) small.push_back(i);
     else if (b->grp[i] == 1 && d >= 4 && d <= 32 && N > from && N <= 22000) mid.push_back(i);
     else rest.push_back(i);
+  }
+  bool levels_pay = from == 8192;
+  for (int i : mid) levels_pay = levels_pay || b->d[i] > 4 || b->N[i] > 10500 || (b->N[i] > 8192 && b->N[i] <= 9500);
+  if (!levels_pay) {
+    rest.insert(rest.end(), mid.begin(), mid.end());
+    mid.clear();
   }
   // The kernels follow one another and each has its tail.  With graphs for the
   // level-by-level teams the split pays (1.0 to 2.1 times); with small

@@ -37,6 +37,13 @@ def test_small_graphs(gpu, n, d, k, kind):
     assert _run(n, d, k)[0] == kind
 
 
+@pytest.mark.parametrize("n,d,k,kind", [(7000, 4, 16, "windows"), (8000, 4, 16, "windows"), (10000, 4, 16, "windows"),
+                                        (8600, 4, 16, "levels"), (11000, 4, 16, "levels"), (10000, 4, 4, "levels"),
+                                        (6000, 6, 16, "levels"), (7000, 5, 16, "levels")])
+def test_mid_size_graphs(gpu, n, d, k, kind):
+    assert _run(n, d, k)[0] == kind
+
+
 @pytest.mark.parametrize("n,k", [(10000, 32), (20000, 8)])
 def test_window_teams_stay_near_l2(gpu, n, k):
     """The teams' matrices of graphs that only windows serve (degree 3)."""
