@@ -328,12 +328,14 @@ double slices_us(const ggb_batch* b) {
   for (const auto& l : b->slices) {
     const int k = l.smem <= 72 * 1024 ? 0 : l.smem <= 110 * 1024 ? 1 : 2;
     const double share = std::min((double)(3 - k), std::max(1.0, (double)l.items / b->sms));
-    double sum = 0.0, last = 0.0;
+    double sum = 0.0, last = 0.0, levels = 0.0, row = 0.0;
     for (int t = l.first; t < l.first + l.items; ++t) {
       const auto& it = b->slice_items[t];
       const int N = b->N[it.graph], pairs = (b->d[it.graph] + 1) / 2, windows = it.end - it.first;
-      const double levels = expected_levels(N, b->d[it.graph]);
-      const double row = (levels - 1.0) * std::pow(4.0 * ((pairs + 1) / 2), 0.7) + 0.5 * levels * pairs;
+      if (it.first == 0) {   // a graph's first item
+        levels = expected_levels(N, b->d[it.graph]);
+        row = (levels - 1.0) * std::pow(4.0 * ((pairs + 1) / 2), 0.7) + 0.5 * levels * pairs;
+      }
       const double gathers = windows * N * row * (l.words == 1 ? 0.6 : 1.0);
       sum += gathers * kGather[k] + windows * levels * kLevel[k] + 4.6e-4 * N * pairs;
       last = std::max(last, gathers * 2.5e-5 * share + 0.23 * windows * levels);
